@@ -295,7 +295,7 @@ struct PathGeo {
     return ADV_STEP;
   }
 
-  template <bool COOP, int PHASE>
+  template <int PHASE>
   __device__ int advance(Hist& h, Stream& g) const {
     const Consts& C = P.C;
     const double eps = kEps64;
@@ -334,7 +334,7 @@ struct PathGeo {
     h.limit = limit;
     if (C.straggling) {
       if constexpr (PHASE == 0) {
-        if (straggled_step<R, COOP, true, true>(m, C, s, Li, R(0), rho, step, g, false, limit,
+        if (straggled_step<R, true, true>(m, C, s, Li, R(0), rho, step, g, false, limit,
                                                 h.x)) {
           h.x.kind = CONT_STRAG;
           h.x.medium = h.med;
@@ -342,7 +342,7 @@ struct PathGeo {
         }
         return step_end(h, h.x.moved);
       } else {
-        if (mixed_step<R, COOP, true>(m, C, s, rho, step, g, limit, h.x)) {
+        if (mixed_step<R, true>(m, C, s, rho, step, g, limit, h.x)) {
           h.x.kind = CONT_MIXED;
           h.x.medium = h.med;
           return ADV_WAIT;
@@ -366,7 +366,7 @@ struct PathGeo {
         mixed_end(h.s, x, Emax, h.limit, false);
       } else {
         ++x.event;
-        if (mixed_run_in<R, true>(m, P.C, h.s, x, g, h.limit)) {
+        if (mixed_run_in<R>(m, P.C, h.s, x, g, h.limit)) {
           x.kind = CONT_MIXED;
           return ADV_WAIT;
         }
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(T, 1) dir_kernel(const __grid_constant__ DirPa
   __syncthreads();
   PathGeo<R> geo{P, meds};
   float* coop = reinterpret_cast<float*>(smem + dir_coop_offset<R>(P));
-  transport_histories<R, PHASE, KCfg<R>::coop>(geo, P.C, P.counter,
+  transport_histories<R, PHASE>(geo, P.C, P.counter,
                                                static_cast<DirHandoff<R>*>(P.queue), coop,
                                                P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
                                                nullptr, ((P.sync >> PHASE) & 1) != 0);
@@ -511,7 +511,7 @@ int dir_launch_t(dp_ctx* ctx, DirParams& P) {
   P.coop_kmax = 1;
   P.coop_kc = 0;
   P.sync = ctx->mc_sync[DP_KERNEL_DIR][sizeof(R) == 4];
-  P.coop_stride = KCfg<R>::coop ? coop_floats(P.coop_nel, 1) : 0;
+  P.coop_stride = coop_warp_floats<R>(P.coop_nel);
   size_t coop_bytes = size_t(warps) * P.coop_stride * sizeof(float);
   int dev_smem = 0;
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
@@ -523,7 +523,7 @@ int dir_launch_t(dp_ctx* ctx, DirParams& P) {
     P.n_staged = k;
     if (dir_coop_offset<R>(P) + coop_bytes <= size_t(dev_smem)) break;
   }
-  if (KCfg<R>::coop) {
+  if (sizeof(R) == 4) {
     // the shared memory left after the staged media, up to the smallest
     // carve-out step that holds a one-event-per-warp buffer, batches DCS sums
     const size_t cap = std::min(size_t(dev_smem), carveout_cap(dir_coop_offset<R>(P) + coop_bytes));
@@ -534,7 +534,7 @@ int dir_launch_t(dp_ctx* ctx, DirParams& P) {
   }
   const size_t smem = dir_coop_offset<R>(P) + coop_bytes;
   if (smem > size_t(dev_smem)) return fail(ctx, DP_ERR_ARG, "too many media for the fixed-path MC kernel");
-  const long need = (P.n + threads - 1) / threads;
+  const long need = sizeof(R) == 4 ? (P.n + threads - 1) / threads : P.n;
   const long rec_blocks = std::min((P.n + 255) / 256, 152L * 32);
   DP_CHECK_CUDA(ctx, cudaMemsetAsync(P.counter, 0, 3 * sizeof(unsigned long long), ctx->stream));
   timed_begin(ctx);

@@ -219,8 +219,11 @@ Layout make_layout(const dp_mixture* const* media, int n_media, size_t esize) {
   }
   L.ld = pad_elems(L.n, esize);
   L.ldk = pad_elems(L.nk, esize);
-  // elements, then the index-table origins and widths (2 doubles per column)
-  L.o_phys = uint32_t((kMaxEl * kElStride + 2 * I_NCOL) * sizeof(double));
+  // elements, then the index-table origins and widths (2 doubles per column),
+  // then (FP64) the elements' DCS constants
+  int nel = 0;
+  for (int k = 0; k < n_media; ++k) nel = std::max(nel, media[k]->nel);
+  L.o_phys = uint32_t((kEldOffset + (esize == 8 ? nel * kEldStride : 0)) * sizeof(double));
   L.o_ker = L.o_phys + uint32_t(size_t(MC_LB1 + 2 * L.slots) * L.ld * esize);
   L.o_idx = L.o_ker + uint32_t(size_t(K_NCOL) * L.ldk * esize);
   L.nbp = kIdxBinsPhys;
@@ -236,6 +239,36 @@ Layout make_layout(const dp_mixture* const* media, int n_media, size_t esize) {
   L.kuniform = L.uniform && a->nk == 8 * (a->n - 1) + 1 && same_nk ? 1 : 0;
   L.kinv_dlE = 8.0 * ph->view.inv_dlE;
   return L;
+}
+
+// The per-element constants of the FP64 DCS sums (src/Materials.jl:576-832).
+static void pack_dcs(const dp_mixture* m, double* out) {
+  const double mm = m->phys->settings.mass * 1e3;  // MeV
+  for (int e = 0; e < m->nel; ++e) {
+    const double* x = m->el.data() + kElStride * e;
+    double* o = out + kEldStride * e;
+    const double Z = x[0], A = x[1], rl = radiation_log(Z), z13 = std::pow(Z, 1.0 / 3.0);
+    const double dn = 1.54 * std::pow(A, 0.27), mu = mm / (kMmuMeV * std::exp(1.0) / dn);
+    const double rho = std::sqrt(1.0 + 4.0 * mu * mu), lr = std::log((rho + 1.0) / (rho - 1.0));
+    const double me_m = kMeMeV / mm, aux = 2.0 * me_m * kReCm * Z;
+    o[EL_Z] = Z;
+    o[EL_A] = A;
+    o[EL_I] = x[2];
+    o[EL_SCALE] = x[3] * kAvogadro / (A * 0.001);
+    o[EL_RLZ] = rl / z13;
+    o[EL_Z13] = z13;
+    o[EL_MDN2] = me_m * dn * (me_m * dn);
+    o[EL_PRE] = rl / z13 / me_m / dn;
+    o[EL_G1] = (Z == 1.0 ? 4.4e-5 : 1.95e-5) * std::pow(Z, 2.0 / 3.0);
+    o[EL_G2] = (Z == 1.0 ? 4.8e-5 : 5.3e-5) * z13;
+    o[EL_LOGA] = std::log(A);
+    o[EL_D1] = (std::log(mu) + 0.5 * rho * lr) * (1.0 - 1.0 / Z);
+    o[EL_D2] = (std::log(mu) + 0.25 * (3.0 * rho - rho * rho * rho) * lr + 2.0 * mu * mu) *
+               (1.0 - 1.0 / Z);
+    o[EL_RLI] = (Z == 1.0 ? 446.0 : 1429.0) / (z13 * z13) * kSqrtE;
+    o[EL_BREMS] = aux * aux * kAlpha * 1e-4;
+    o[EL_CPF] = 4.0 / (3.0 * kPi) * Z * (kAlpha * kReCm) * (kAlpha * kReCm);
+  }
 }
 
 template <class R>
@@ -266,6 +299,7 @@ static void pack(const dp_mixture* m, const Layout& L, unsigned char* out) {
     f[4] = float(kAvogadro / (x[1] * 0.001));
     f[5] = float(x[4]);  // nuclear RMS radius (DEL polar angles)
   }
+  if (sizeof(R) == 8) pack_dcs(m, reinterpret_cast<double*>(out) + kEldOffset);
   // index tables of the inverse lookups (origins and widths in R)
   R* prm = reinterpret_cast<R*>(reinterpret_cast<double*>(out) + kMaxEl * kElStride);
   int16_t* idx = reinterpret_cast<int16_t*>(out + L.o_idx);
@@ -564,9 +598,9 @@ struct SlabGeo {
   // the descriptors by medium index: rock and air are consecutive entries of
   // the CTA's descriptor array in shared memory
   __device__ const Med<R>* media() const { return &rock; }
-  template <bool COOP, int PHASE>
+  template <int PHASE>
   __device__ int advance(Hist& h, Stream& g) const {
-    return mc::advance<R, COOP, PHASE>(rock, air, nullptr, P.C, h, g);
+    return mc::advance<R, PHASE>(rock, air, nullptr, P.C, h, g);
   }
   template <int PHASE>
   __device__ int resume(Hist& h, Stream& g) const {
@@ -605,9 +639,9 @@ struct SlabGeoP {
   __device__ const Med<R>& medium(int k) const { return k == 1 ? air : (k == 2 ? porous : rock); }
   // rock, air and porous are consecutive entries of the CTA's descriptor array
   __device__ const Med<R>* media() const { return &rock; }
-  template <bool COOP, int PHASE>
+  template <int PHASE>
   __device__ int advance(Hist& h, Stream& g) const {
-    return mc::advance<R, COOP, PHASE>(rock, air, &porous, P.C, h, g);
+    return mc::advance<R, PHASE>(rock, air, &porous, P.C, h, g);
   }
   template <int PHASE>
   __device__ int resume(Hist& h, Stream& g) const {
@@ -657,14 +691,14 @@ __global__ void __launch_bounds__(T, 1) mc_kernel(const __grid_constant__ McPara
   if constexpr (POR) {
     const Med<R>& porous = meds[2];
     SlabGeoP<R> geo{P, rock, air, porous};
-    transport_histories<R, PHASE, KCfg<R>::coop>(geo, P.C, P.counter,
+    transport_histories<R, PHASE>(geo, P.C, P.counter,
                                                  static_cast<HandoffP<R>*>(P.queue), coop,
                                                  P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
                                                  PHASE == 0 ? P.order0 : P.order1,
                                                  ((P.sync >> PHASE) & 1) != 0);
   } else {
     SlabGeo<R> geo{P, rock, air};
-    transport_histories<R, PHASE, KCfg<R>::coop>(geo, P.C, P.counter,
+    transport_histories<R, PHASE>(geo, P.C, P.counter,
                                                  static_cast<Handoff<R>*>(P.queue), coop,
                                                  P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
                                                  PHASE == 0 ? P.order0 : P.order1,
@@ -1005,7 +1039,7 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
   P.coop_kmax = 1;
   P.coop_kc = 0;
   P.sync = ctx->mc_sync[DP_KERNEL_MC][sizeof(R) == 4];
-  P.coop_stride = KCfg<R>::coop ? coop_floats(P.coop_nel, 1) : 0;
+  P.coop_stride = coop_warp_floats<R>(P.coop_nel);
   size_t coop_bytes = size_t(warps) * P.coop_stride * sizeof(float);
   size_t tables = size_t(POR ? 3 : 2) * P.lay.med_bytes;
   int dev_smem = 0;
@@ -1017,7 +1051,7 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
   // the shared memory left after the tables (up to `cap` bytes in all)
   // batches DCS sums
   auto fit = [&](size_t cap) -> size_t {
-    if (KCfg<R>::coop) {
+    if (sizeof(R) == 4) {
       const size_t used = mc_smem_head<R>() + (P.staged ? tables : 0);
       P.coop_kmax = coop_kmax(cap - std::min(cap, used), warps, P.coop_nel);
       P.coop_stride = coop_floats(P.coop_nel, P.coop_kmax);
@@ -1031,7 +1065,7 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
   // the DCS buffer fills the smallest carve-out step that holds it, the rest
   // of the SM's 256 KB is L1 for the spilled stack
   smem = fit(std::min(size_t(dev_smem), carveout_cap(smem)));
-  long need = (P.n + threads - 1) / threads;
+  long need = sizeof(R) == 4 ? (P.n + threads - 1) / threads : P.n;
   long rec_blocks = std::min((P.n + 255) / 256, 152L * 32);
   DP_CHECK_CUDA(ctx, cudaMemsetAsync(P.counter, 0, 3 * sizeof(unsigned long long), ctx->stream));
   timed_begin(ctx);

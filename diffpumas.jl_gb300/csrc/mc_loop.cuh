@@ -12,7 +12,7 @@
 //   void end(long i, const Hist&)             end record of history i
 //   const Med<R>& medium(int k) const         medium of a suspended step
 //   const Med<R>* media() const               the descriptors by medium index
-//   int advance<COOP, PHASE>(Hist&, Stream&)  one step: ADV_*
+//   int advance<PHASE>(Hist&, Stream&)        one step: ADV_*
 //   int resume<PHASE>(Hist&, Stream&)         finish a suspended step: ADV_*
 #pragma once
 #include <cooperative_groups.h>
@@ -33,15 +33,13 @@ namespace mc {
 // (dp_set_mc_threads, dp_autotune).  The transport is latency bound, so the
 // most warps win: 1024 threads run the two-layer and fixed-path workloads
 // 1.3-1.4x faster than 512, with 164 bytes of spills.  The FP64 transport
-// (one thread per sum, 255 registers) runs 8 warps.
+// (255 registers) runs 8 warps.
 template <class R> struct KCfg;
 template <> struct KCfg<float> {
   static constexpr int threads = 1024;  // default CTA size
-  static constexpr bool coop = true;
 };
 template <> struct KCfg<double> {
   static constexpr int threads = 256;
-  static constexpr bool coop = false;
 };
 
 // Calls f(std::integral_constant<int, T>{}) with T the compiled CTA size
@@ -84,6 +82,11 @@ inline int carveout_percent(int device, size_t smem) {
   return pct < 0 ? 0 : (pct > 100 ? 100 : pct);
 }
 
+// Floats of one warp's least DCS buffer: one event (FP64: its doubles).
+template <class R>
+inline int coop_warp_floats(int nel) {
+  return sizeof(R) == 4 ? coop_floats(nel, 1) : 2 * ((del64_doubles(nel) + 1) & ~1);
+}
 // Events a warp's batched DCS pass serves at once: as many as `avail` bytes of
 // shared memory hold for `warps` warps, between 1 and 32 (a warp's lanes).
 inline int coop_kmax(size_t avail, int warps, int nel) {
@@ -266,16 +269,34 @@ __device__ __forceinline__ void serve_cta(const G& geo, const Consts& C, float* 
   }
 }
 
+// Whether this thread of the FP64 transport takes histories, for n of them on
+// a grid of `warps` warps.  An FP64 warp instruction holds its SM partition for
+// 64 cycles with one lane active as with 32 (measured), so a lane alone in its
+// warp costs as much as a full warp, but a history's divergent paths (hard
+// events, rejection loops) then wait for no other lane and no other warp.  So
+// the histories are spread over all warps of the grid, first one warp of every
+// CTA, then the next, and lanes are filled once every warp has one.
+// run_backward_mc, 100 m of rock: 10^3 histories 64.7 -> 37.9 ms, 10^4 78.5 ->
+// 67.0 ms against full warps on the fewest CTAs; a direction of 256 histories
+// 40.3 -> 13.3 ms.  At 10^5 histories all lanes are full and both are equal.
+__device__ __forceinline__ bool fp64_takes(long n, int lane) {
+  const long warps = long(gridDim.x) * (blockDim.x >> 5);
+  const long l = n <= warps ? 1 : (n + warps - 1) / warps;
+  const long rank = long(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  return l >= 32 || (lane < l && rank * l + lane < n);
+}
+
 // Runs histories until none is left for this phase.  counter[PHASE] hands out
-// history indices, counter[2] counts the hand-off queue.  With COOP, `coop`
-// is the CTA's shared memory for batched DCS sums: per warp `stride` floats
-// (coop_floats for up to kmax events of one medium), or, in lockstep, one
-// CTA buffer (cta_floats(nel, kc)).  `order` (may be null) maps the j-th
+// history indices, counter[2] counts the hand-off queue.  `coop` is the CTA's
+// shared memory for DCS sums.  FP32: per warp `stride` floats (coop_floats for
+// up to kmax events of one medium), or, in lockstep, one CTA buffer
+// (cta_floats(nel, kc)).  FP64: per warp `stride` floats, del64_doubles(nel)
+// doubles among them.  `order` (may be null) maps the j-th
 // hand-out to a history (phase 0) or a queue slot (phase 1): the
 // longest-first schedule.  With `lockstep` (block-uniform) every warp of the
 // CTA runs its loop iterations in step with the others until the CTA has no
 // history left, and the CTA serves all its waiting steps together.
-template <class R, int PHASE, bool COOP, class G>
+template <class R, int PHASE, class G>
 __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
                                                     unsigned long long* counter,
                                                     typename G::Queue* queue, float* coop,
@@ -311,8 +332,8 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
     return true;
   };
   long i = 0;
-  bool live = take(&i);
-  if constexpr (COOP) {
+  if constexpr (sizeof(R) == 4) {
+    bool live = take(&i);
     if (lockstep && kc > 0) {
       int* cnt = reinterpret_cast<int*>(coop);
       if (threadIdx.x == 0) cnt[0] = cnt[1] = 0;
@@ -323,7 +344,7 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
         serve_cta(geo, C, coop, kc, nel, parity, live && h.x.kind != CONT_NONE, h.x, g);
         if (live) {
           const int r = h.x.kind != CONT_NONE ? geo.template resume<PHASE>(h, g)
-                                              : geo.template advance<true, PHASE>(h, g);
+                                              : geo.template advance<PHASE>(h, g);
           live = settle(r, &i);
         }
         if (!__syncthreads_or(live)) break;
@@ -378,13 +399,53 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
       }
       if (live) {
         const int r = h.x.kind != CONT_NONE ? geo.template resume<PHASE>(h, g)
-                                            : geo.template advance<true, PHASE>(h, g);
+                                            : geo.template advance<PHASE>(h, g);
         live = settle(r, &i);
       }
       if (!__any_sync(0xffffffffu, live)) break;
     }
   } else {
-    while (live) live = settle(geo.template advance<false, PHASE>(h, g), &i);
+    // FP64: the warp serves its waiting lanes one event at a time, all lanes
+    // on the terms of the event's sum (del64_sum)
+    const int lane = threadIdx.x & 31;
+    double* buf = reinterpret_cast<double*>(coop + size_t(threadIdx.x >> 5) * stride);
+    bool live = fp64_takes(n, lane) && take(&i);
+    while (__any_sync(0xffffffffu, live)) {
+      unsigned want = __ballot_sync(0xffffffffu, live && h.x.kind != CONT_NONE);
+      while (want) {
+        const int from = __ffs(want) - 1;
+        want &= want - 1;
+        const Med<R>& m = geo.medium(__shfl_sync(0xffffffffu, h.x.medium, from));
+        const double anc = __shfl_sync(0xffffffffu, h.x.anc, from);
+        const double q = __shfl_sync(0xffffffffu, h.x.q, from);
+        const double total = del64_sum(m.el + kEldOffset, m.nel, C.mass, anc, q, buf);
+        if (lane == from) {
+          h.x.total = total;
+          h.x.pick = -1;
+          if (h.x.details && total > 0.0) {
+            // process and element pick in the reference's order (src/MixedTransport.jl:131-140)
+            const double* comp = buf + 12 * kPairPt + 9 * kPhotoPt + m.nel;
+            const int last = 4 * m.nel - 1;
+            double u = uni<R>(g) * total;
+            int pick = last;
+            for (int c = 0; c <= last; ++c) {
+              u -= comp[c];
+              if (u <= 0.0) {
+                pick = c;
+                break;
+              }
+            }
+            h.x.pick = pick;
+          }
+        }
+        __syncwarp();
+      }
+      if (live) {
+        const int r = h.x.kind != CONT_NONE ? geo.template resume<PHASE>(h, g)
+                                            : geo.template advance<PHASE>(h, g);
+        live = settle(r, &i);
+      }
+    }
   }
 }
 
