@@ -1,0 +1,113 @@
+// fp64_math.cuh -- FP64 elementary functions for the walks of this library.
+//
+// GB300 issues one FP64 warp instruction per 64 cycles and SM partition, so the
+// FP64 kernels are bound by the number of those instructions and by nothing
+// else.  Measured (cycles of one warp, dependent calls): log 2087, exp 1334,
+// a / b 641, sqrt 676, sincospi 1948, against 64 for one multiply-add.  The
+// forms below trade arithmetic for small tables and integer work, which runs on
+// other pipes:
+//  - log and exp after the table-driven scheme of P. T. P. Tang (ACM TOMS 15,
+//    1989 and 16, 1990): the argument's leading bits select a tabulated value,
+//    a short Taylor polynomial of the small remainder does the rest;
+//  - the reciprocal and the reciprocal square root refine the hardware's
+//    approximation by the binomial series of its residual;
+//  - comparisons, minima and uniforms on the bit patterns.
+// All are within 1.5 units in the last place (division: 2) of the exact value
+// on the ranges that the walks use (tested against CUDA's functions); outside
+// them (zeros, negative or subnormal arguments, infinities, NaN) they call
+// CUDA's.
+#pragma once
+#include <stdint.h>
+
+#include "common.cuh"
+
+namespace dp {
+namespace f64 {
+
+#include "fp64_tables.inc"
+
+__device__ __forceinline__ int hi32(double x) { return __double2hiint(x); }
+// The integer k as a double: one subtraction instead of a conversion.
+__device__ __forceinline__ double from_int(int k) {
+  return __hiloint2double(0x43300000, int(uint32_t(k) ^ 0x80000000u)) - 4503601774854144.0;
+}
+
+// log x, x normal and positive: 10 FP64 instructions.  x = 2^k m with m / c in
+// [1 - 2^-9, 1 + 2^-9] of the table's c; c = 1 around x = 1, where the result
+// is the polynomial alone.
+__device__ __forceinline__ double log(double x) {
+  const int hi = hi32(x);
+  if (uint32_t(hi - 0x00100000) >= 0x7fe00000u) return ::log(x);
+  const int k = ((hi + 0x00080800) >> 20) - 1023;
+  const double2 t = kLogTab[((hi & 0xfffff) + 0x800) >> 12];
+  const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
+  const double r = fma(m, t.x, -1.0);
+  const double p = fma(r, fma(r, fma(r, fma(r, -1.0 / 6.0, 0.2), -0.25), 1.0 / 3.0), -0.5);
+  return fma(from_int(k), 0.6931471805599453, t.y) + fma(r * r, p, r);
+}
+
+// exp x: 10 FP64 instructions; x = (128 k + j) log 2 / 128 + r, |r| <= log 2 / 256.
+__device__ __forceinline__ double exp(double x) {
+  if (uint32_t(hi32(x) & 0x7fffffff) >= 0x40862000u) return ::exp(x);  // |x| >= 708
+  const double s = fma(x, 184.6649652337873, 6755399441055744.0);  // 1.5 2^52: nearest integer
+  const int n = __double2loint(s);
+  const double d = s - 6755399441055744.0;
+  const double r = fma(d, -1.2864023111638346e-14, fma(d, -0.005415212348111709, x));
+  const double p = fma(r, fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
+  const double t = kExpTab[n & 127], y = fma(t, r * p, t);
+  return __hiloint2double(hi32(y) + ((n >> 7) << 20), __double2loint(y));
+}
+
+// 1 / x for normal x whose reciprocal is normal: 3 FP64 instructions.
+__device__ __forceinline__ double rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double div(double a, double b) { return a * rcp(b); }
+
+// 1 / sqrt(x) and sqrt(x) for normal positive x: 5 and 6 FP64 instructions.
+__device__ __forceinline__ double rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double sqrt(double x) { return x > 0.0 ? x * rsqrt(x) : ::sqrt(x); }
+
+// sin(pi x) and cos(pi x) for |x| <= 1: 18 FP64 instructions; the nearest
+// multiple of 1/32 from the table and quadrant symmetry, the remainder
+// |d| <= pi / 64 by Taylor polynomials.
+__device__ __forceinline__ void sincospi(double x, double* sn, double* cs) {
+  const double s = fma(x, 32.0, 6755399441055744.0);
+  const int n = __double2loint(s) & 63;
+  const double d = fma(s - 6755399441055744.0, -0.03125, x) * kPi, d2 = d * d;
+  const double sd = fma(d * d2, fma(d2, fma(d2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), d);
+  const double cd = d2 * fma(d2, fma(d2, fma(d2, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5);  // cos d - 1
+  const int q = n >> 4, j = n & 15;
+  const double2 t = kSinTab[j];
+  const double a = fma(t.x, cd, fma(t.y, sd, t.x)), b = fma(t.y, cd, fma(-t.x, sd, t.y));
+  // quadrant q of pi/2: (sin, cos) -> (cos, -sin) ...
+  const double u = (q & 1) ? b : a, v = (q & 1) ? a : b;
+  *sn = __hiloint2double(hi32(u) ^ ((q & 2) << 30), __double2loint(u));
+  *cs = __hiloint2double(hi32(v) ^ (((q + 1) & 2) << 30), __double2loint(v));
+}
+
+// a < b for non-negative a and b (or both NaN-free and of one order by bits).
+__device__ __forceinline__ bool lt_pos(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ double min_pos(double a, double b) { return lt_pos(b, a) ? b : a; }
+__device__ __forceinline__ double max_pos(double a, double b) { return lt_pos(a, b) ? b : a; }
+
+// u01 on the bit pattern: m 2^-53 of the 53-bit integer m, no FP64 instruction.
+__device__ __forceinline__ double uniform(uint32_t a, uint32_t b) {
+  const uint64_t m = (uint64_t(a >> 5) << 26) | uint64_t(b >> 6);
+  if (m == 0) return 0.0;
+  const int z = __clzll(m);  // 11 ... 63
+  return __longlong_as_double((m << (z - 11) & 0xfffffffffffffull) | (uint64_t(1033 - z) << 52));
+}
+
+}  // namespace f64
+}  // namespace dp

@@ -2,8 +2,8 @@
 // the device: compute_directional_flux_csda (:667-727),
 // directional_flux_and_grad_csda and assemble_forward_and_jacobian
 // (:736-820), with the CSDA correction multipliers (:85-214, :367-412,
-// :557-579).  Two instances of the walk (wtomo_walk.cuh): FP64, the
-// reference's operations, and mixed precision, FP32 steps and tangents with
+// :557-579).  Two instances of the walk: FP64 (wtomo_fp64.cuh), the
+// reference's operations, and mixed precision (wtomo_walk.cuh), FP32 steps and tangents with
 // the adjoint's prefix sums, the flux and the reductions in FP64.
 //
 // One warp per direction, one lane per energy sample.  d flux / d w comes from
@@ -25,6 +25,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fp64_math.cuh"
 #include "internal.h"
 
 namespace dp {
@@ -115,16 +116,8 @@ __device__ __forceinline__ double warp_sum(double x) {
 }  // namespace wt
 }  // namespace dp
 
-#define WT_NS wt64
-#define WT_REAL double
+#include "wtomo_fp64.cuh"
 #include "wtomo_walk.cuh"
-#undef WT_NS
-#undef WT_REAL
-#define WT_NS wt32
-#define WT_REAL float
-#include "wtomo_walk.cuh"
-#undef WT_NS
-#undef WT_REAL
 
 namespace {
 
@@ -206,20 +199,22 @@ int run(dp_ctx* ctx, const dp_physics* ph, const dp_csda_config* c, const dp_csd
   if (precision != DP_PREC_FP64 && precision != DP_PREC_MIXED)
     return fail(ctx, DP_ERR_ARG, "precision must be DP_PREC_FP64 or DP_PREC_MIXED");
   const bool mixed = precision == DP_PREC_MIXED;
-  // FP64 columns staged, plus their FP32 copy for the mixed instance
-  const size_t smem = 16 + size_t(wt::kSlots) * P.col_bytes * (mixed ? 3 : 2) / 2;
+  // the staged FP64 columns with their FP32 copy (mixed), or with the columns
+  // the FP64 walk derives
+  const size_t smem = 16 + (mixed ? size_t(wt::kSlots) * P.col_bytes * 3 / 2
+                                  : size_t(wt64::kCols) * P.col_bytes);
+  const int threads = mixed ? wt::kThreads : wt64::kThreads;
   auto kernel = mixed ? wt32::wtomo_kernel : wt64::wtomo_kernel;
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           int(smem)));
   int per_sm = 0, n_sm = 0;
-  DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, wt::kThreads,
-                                                                   smem));
+  DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-  const long need = (B->n_bins + wt::kThreads / 32 - 1) / (wt::kThreads / 32);
+  const long need = (B->n_bins + threads / 32 - 1) / (threads / 32);
   const long blocks = std::max(1L, std::min(need, long(std::max(per_sm, 1)) * n_sm));
   DP_CHECK_CUDA(ctx, cudaMemsetAsync(P.next_bin, 0, sizeof(unsigned long long), ctx->stream));
   timed_begin(ctx);
-  kernel<<<int(blocks), wt::kThreads, smem, ctx->stream>>>(P);
+  kernel<<<int(blocks), threads, smem, ctx->stream>>>(P);
   DP_CHECK_CUDA(ctx, cudaGetLastError());
   timed_end(ctx, mixed ? (jac ? "dir_csda32_grad" : "dir_csda32") : (jac ? "dir_csda_grad" : "dir_csda"));
   return DP_OK;

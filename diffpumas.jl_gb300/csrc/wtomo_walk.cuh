@@ -1,13 +1,11 @@
-// wtomo_walk.cuh -- the CSDA walk and the kernel of wtomo.cu in one scalar
-// type.  wtomo.cu includes it twice: WT_REAL double (the reference's FP64
-// operations) and WT_REAL float (FP32 steps and tangents; the prefix sums of
-// the adjoint, the flux and the reductions stay FP64).  No include guard on
-// purpose; WT_NS names the namespace of each instance.
+// wtomo_walk.cuh -- the mixed-precision instance of the CSDA walk and its
+// kernel (wtomo.cu): FP32 steps and tangents as dual numbers; the prefix sums
+// of the adjoint, the flux and the reductions stay FP64.
 
 namespace dp {
-namespace WT_NS {
+namespace wt32 {
 
-using Real = WT_REAL;
+using Real = float;
 using wt::Lane;
 using wt::Params;
 using wt::kMaxChunks;
@@ -356,17 +354,12 @@ __device__ Lane pass1(const Params& P, const Consts& k, const Tables& tb, long b
   return out;
 }
 
-// Copies the staged FP64 columns into the walk's precision (FP32 instance) or
-// uses them in place (FP64 instance).
+// Copies the staged FP64 columns into the walk's precision.
 __device__ __forceinline__ const Real* convert_columns(double* cols, unsigned char* spare, int count) {
-  if constexpr (sizeof(Real) == 8) {
-    return reinterpret_cast<const Real*>(cols);
-  } else {
-    Real* out = reinterpret_cast<Real*>(spare);
-    for (int i = threadIdx.x; i < count; i += blockDim.x) out[i] = Real(cols[i]);
-    __syncthreads();
-    return out;
-  }
+  Real* out = reinterpret_cast<Real*>(spare);
+  for (int i = threadIdx.x; i < count; i += blockDim.x) out[i] = Real(cols[i]);
+  __syncthreads();
+  return out;
 }
 
 __global__ void __launch_bounds__(kThreads) wtomo_kernel(const __grid_constant__ Params P) {
@@ -509,5 +502,5 @@ __global__ void __launch_bounds__(kThreads) wtomo_kernel(const __grid_constant__
   }
 }
 
-}  // namespace WT_NS
+}  // namespace wt32
 }  // namespace dp
