@@ -174,6 +174,7 @@ struct dp_paths {
   int32_t* perm = nullptr;      // entries sorted by (cell, entry index)
   float4* geom = nullptr;       // per ray: cos_theta_star, its 1.29 power,
                                 // 1/max(|cos theta|, 0.01), cos theta
+  double2* star = nullptr;      // per ray: cos_theta_star and its 1.29 power in FP64
   int32_t* order = nullptr;     // rays by decreasing segment count (schedule)
   int32_t* prow = nullptr;      // row_of[perm[p]] (gather reads it in order)
   int32_t* big = nullptr;       // cells whose bucket holds more than 32 entries

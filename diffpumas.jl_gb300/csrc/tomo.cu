@@ -35,6 +35,7 @@
 #include <string>
 #include <vector>
 
+#include "fp64_math.cuh"
 #include "internal.h"
 
 namespace dp {
@@ -132,13 +133,15 @@ __device__ __forceinline__ int trace(const GridDev& g, const dp_ray& r, int cap,
 // One thread per ray: segments into a fixed-capacity slot, count per ray.
 __global__ void trace_kernel(GridDev g, const dp_ray* rays, long n_rays, int cap, int side_cell,
                              int32_t* slot_cell, double* slot_len, int64_t* counts,
-                             float4* geom, int* err_flag) {
+                             float4* geom, double2* star, int* err_flag) {
   long r = blockIdx.x * long(blockDim.x) + threadIdx.x;
   if (r >= n_rays) return;
   dp_ray ray = rays[r];
   {
     double cs = cos_theta_star(ray.cos_theta);
-    geom[r] = make_float4(float(cs), float(pow(cs, 1.29)),
+    const double cs129 = pow(cs, 1.29);
+    star[r] = double2{cs, cs129};
+    geom[r] = make_float4(float(cs), float(cs129),
                           float(1.0 / fmax(fabs(ray.cos_theta), 0.01)), float(ray.cos_theta));
   }
   int32_t* sc = slot_cell + size_t(r) * cap;
@@ -329,6 +332,8 @@ struct EvalP {
   TabView tab;
   const float* tab32;
   const float4* geom;
+  const double2* star;  // per ray: cos_theta_star and its 1.29 power
+  double2* work;        // FP64 adjoint: per resident warp, segment and lane
   const NodeInit* node0;
   const int32_t* order;
   int ld32;
@@ -352,153 +357,15 @@ __device__ __forceinline__ double seg_density(const EvalP& P, int c) {
   return c >= 0 ? P.rho[c] : P.side_density;
 }
 
-// d log D / d Eavg, D = exp(-L/(beta gamma ctau)), beta = sqrt(max(1-1/g^2, 1e-12))
-__device__ __forceinline__ double decay_log(double L, double Eavg, double mass, double ctau,
-                                            double* dlog) {
-  double g = 1.0 + Eavg / mass, b2 = 1.0 - 1.0 / (g * g);
-  bool clamp = !(b2 > 1e-12);
-  double b = sqrt(clamp ? 1e-12 : b2), bg = b * g;
-  if (dlog) *dlog = L / (ctau * bg * bg) * (clamp ? b : 1.0 / b) / mass;
-  return -L / (bg * ctau);
-}
-__device__ __forceinline__ double dlogS(const TabView& t, const double* E, const double* lE,
-                                        const double* S, double e) {
-  Dd s = interp_logE(t, E, lE, S, dd(e, 1.0 / e), dd(log(e), 1.0 / e), nullptr);
-  return s.d / s.v;
-}
-__device__ __forceinline__ double range_slope(const TabView& t, const double* E, const double* lE,
-                                              const double* R, double e) {
-  return interp_logE(t, E, lE, R, dd(e, 1.0), dd(log(e), 1.0 / e), nullptr).d;
-}
-__device__ __forceinline__ double inv_slope(const double* R, const double* E, const double* lE,
-                                            int n, double Y) {
-  return inverse_range(R, E, lE, n, dd(Y, 1.0), nullptr).d;
+// log D, D = exp(-L/(beta gamma ctau)), beta = sqrt(max(1-1/g^2, 1e-12))
+__device__ __forceinline__ double decay_log(double L, double Eavg, double mass, double ctau) {
+  const double g = 1.0 + Eavg / mass, b2 = 1.0 - 1.0 / (g * g);
+  return -L / (sqrt(b2 > 1e-12 ? b2 : 1e-12) * g * ctau);
 }
 
-enum { T_E = 0, T_LOGE, T_RS, T_RR, T_AS, T_AR, T_NCOL };
 constexpr int kWarps = 4;
 
-// ---------------------------------------------------------------- FP64 kernel
-template <bool ADJ>
-__global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
-  extern __shared__ __align__(16) double smem[];
-  __shared__ uint64_t mbar;
-  const int ld = P.tab.ld, n = P.tab.n;
-  const double* src[T_NCOL] = {P.tab.col(0, DP_COL_E),          P.tab.col(0, DP_COL_LOGE),
-                               P.tab.col(P.rock, DP_COL_CSDA_S), P.tab.col(P.rock, DP_COL_CSDA_R),
-                               P.tab.col(P.air, DP_COL_CSDA_S),  P.tab.col(P.air, DP_COL_CSDA_R)};
-  if (!stage_columns(smem, src, T_NCOL, uint32_t(ld * sizeof(double)), &mbar, P.wait_iters)) {
-    if (threadIdx.x == 0) atomicExch(P.err_flag, 1);
-    return;
-  }
-  const double *tE = smem + T_E * ld, *tlE = smem + T_LOGE * ld;
-  const double *rS = smem + T_RS * ld, *rR = smem + T_RR * ld;
-  const double *aS = smem + T_AS * ld, *aR = smem + T_AR * ld;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = P.seg_cap;
-  double* sL = smem + T_NCOL * ld + size_t(warp) * cap * 3;
-  double* sD = sL + cap;
-  double* sJ = sD + cap;
-  const double Emax = tE[n - 1];
-  for (long q = blockIdx.x * long(kWarps) + warp; q < P.n_rays; q += long(gridDim.x) * kWarps) {
-    const long r = P.order[q];
-    const int64_t off = P.row_ptr[r];
-    const int nseg = int(P.row_ptr[r + 1] - off);
-    for (int s = lane; s < nseg; s += 32) {
-      sL[s] = P.len[off + s];
-      sD[s] = seg_density(P, P.cell[off + s]);
-      sJ[s] = 0.0;
-    }
-    __syncwarp();
-    const double cosz = P.rays[r].cos_theta;
-    const double cs_safe = fmax(fabs(cosz), 0.01);
-    const double Lair = (P.H - P.zmax) / cs_safe;
-    const double Gair = fmax((1.205 * 12e3 / cs_safe) * P.air_dexp, 0.0);
-    const double cs = cos_theta_star(cosz), cs129 = pow(cs, 1.29);
-    double fsum = 0.0;
-    for (int base = 0; base < P.n_nodes; base += 32) {
-      const int nd = base + lane;
-      const bool active = nd < P.n_nodes;
-      double E = active ? P.nE[nd] : 1.0, w = 1.0;
-      bool ok = active;
-      int kc = -1, hint = 0;
-      double Eprev_c = 0.0;
-      for (int s = 0; s < nseg && ok; ++s) {
-        double X = interp_logE(P.tab, tE, tlE, rR, dd(E), dd(log(E)), nullptr).v;
-        double Ek = inverse_range(rR, tE, tlE, n, dd(X + sL[s] * sD[s]), &hint).v;
-        if (!(Ek < 1e12)) {
-          ok = false;
-          break;
-        }
-        if (kc < 0 && Ek >= Emax) {
-          kc = s;
-          Eprev_c = E;
-        }
-        double Si = interp_logE(P.tab, tE, tlE, rS, dd(E), dd(log(E)), nullptr).v;
-        double Sf = interp_logE(P.tab, tE, tlE, rS, dd(Ek), dd(log(Ek)), nullptr).v;
-        w = w * (Sf / Si);
-        w = w * exp(decay_log(sL[s], (E + Ek) / 2.0, P.mass, P.ctau, nullptr));
-        E = Ek;
-      }
-      double f = 0.0, EN = E, Ef = 0.0;
-      if (ok) {
-        double Xa = interp_logE(P.tab, tE, tlE, aR, dd(E), dd(log(E)), nullptr).v;
-        Ef = inverse_range(aR, tE, tlE, n, dd(Xa + Gair), nullptr).v;
-        double Sa0 = interp_logE(P.tab, tE, tlE, aS, dd(E), dd(log(E)), nullptr).v;
-        double Sa1 = interp_logE(P.tab, tE, tlE, aS, dd(Ef), dd(log(Ef)), nullptr).v;
-        w = w * (Sa1 / Sa0);
-        w = w * exp(decay_log(Lair, (E + Ef) / 2.0, P.mass, P.ctau, nullptr));
-        f = w * gccly_flux(cs, cs129, Ef, P.nq[nd], nullptr);
-      }
-      const double coef = ok ? 2.0 * P.nw[nd] / P.n_nodes : 0.0;
-      fsum += coef * f;
-      if (ADJ) {
-        const bool live = coef != 0.0 && f != 0.0;
-        double lam = 0.0;
-        if (live) {
-          double aA, dlogF;
-          decay_log(Lair, (EN + Ef) / 2.0, P.mass, P.ctau, &aA);
-          gccly_flux(cs, cs129, Ef, P.nq[nd], &dlogF);
-          double dEf = inv_slope(aR, tE, tlE, n,
-                                 interp_logE(P.tab, tE, tlE, aR, dd(EN), dd(log(EN)), nullptr).v + Gair) *
-                       range_slope(P.tab, tE, tlE, aR, EN);
-          lam = dlogS(P.tab, tE, tlE, rS, EN) - dlogS(P.tab, tE, tlE, aS, EN) + 0.5 * aA +
-                dEf * (dlogS(P.tab, tE, tlE, aS, Ef) + 0.5 * aA + dlogF);
-        }
-        double Ek = EN;
-        for (int s = nseg - 1; s >= 0; --s) {
-          double v = 0.0, Ekm1 = 0.0;
-          if (live) {
-            const double L = sL[s];
-            if (kc >= 0 && s > kc) {
-              Ekm1 = Emax;
-            } else if (s == kc) {
-              Ekm1 = Eprev_c;
-            } else {
-              double Y = interp_logE(P.tab, tE, tlE, rR, dd(Ek), dd(log(Ek)), nullptr).v;
-              Ekm1 = s == 0 ? P.nE[nd] : inverse_range(rR, tE, tlE, n, dd(Y - L * sD[s]), nullptr).v;
-            }
-            double Ycur = interp_logE(P.tab, tE, tlE, rR, dd(Ekm1), dd(log(Ekm1)), nullptr).v + L * sD[s];
-            double Kp = (Ek >= Emax) ? 0.0 : inv_slope(rR, tE, tlE, n, Ycur);
-            double a;
-            decay_log(L, (Ekm1 + Ek) / 2.0, P.mass, P.ctau, &a);
-            lam += 0.5 * a;
-            v = coef * f * lam * Kp * L;
-            lam = lam * Kp * range_slope(P.tab, tE, tlE, rR, Ekm1) + 0.5 * a;
-          }
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) sJ[s] += v;
-          Ek = Ekm1;
-        }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
-    if (lane == 0) P.flux[r] = fsum;
-    __syncwarp();
-    if (ADJ)
-      for (int s = lane; s < nseg; s += 32) P.jval64[off + s] = sJ[s];
-    __syncwarp();
-  }
-}
+#include "tomo_fp64.cuh"
 
 // ---------------------------------------------------------------- mixed kernel
 // Node start from the FP64 tables (each block computes all nodes once).
@@ -779,7 +646,7 @@ __global__ void plain_ray_kernel(EvalP P, GridDev g, int side_cell, long r, doub
     }
     w *= interp_logE(tb, E_, lE, rS, dd(Ek), dd(log(Ek)), nullptr).v /
          interp_logE(tb, E_, lE, rS, dd(E), dd(log(E)), nullptr).v;
-    w *= exp(decay_log(L, (E + Ek) / 2.0, P.mass, P.ctau, nullptr));
+    w *= exp(decay_log(L, (E + Ek) / 2.0, P.mass, P.ctau));
     E = Ek;
   };
   trace(g, ray, 1 << 30, &z_exit, [&](int, int cell, double L) { seg(P.rho[cell], L); });
@@ -793,7 +660,7 @@ __global__ void plain_ray_kernel(EvalP P, GridDev g, int side_cell, long r, doub
     double Ef = inverse_range(aR, E_, lE, t.n, dd(Xa + Gair), nullptr).v;
     w *= interp_logE(tb, E_, lE, aS, dd(Ef), dd(log(Ef)), nullptr).v /
          interp_logE(tb, E_, lE, aS, dd(E), dd(log(E)), nullptr).v;
-    w *= exp(decay_log((P.H - g.zmax) / cs_safe, (E + Ef) / 2.0, P.mass, P.ctau, nullptr));
+    w *= exp(decay_log((P.H - g.zmax) / cs_safe, (E + Ef) / 2.0, P.mass, P.ctau));
     double cs = cos_theta_star(ray.cos_theta);
     f = w * gccly_flux(cs, pow(cs, 1.29), Ef, P.nq[nd], nullptr);
   }
@@ -842,7 +709,7 @@ static T* dalloc(std::vector<void*>& keep, size_t n) {
 static void free_paths_arrays(dp_paths* p) {
   if (!p->owned) return;
   for (void* x : {(void*)p->rays, (void*)p->row_ptr, (void*)p->cell, (void*)p->len,
-                  (void*)p->row_of, (void*)p->cptr, (void*)p->perm, (void*)p->geom,
+                  (void*)p->row_of, (void*)p->cptr, (void*)p->perm, (void*)p->geom, (void*)p->star,
                   (void*)p->order, (void*)p->prow, (void*)p->big})
     if (x) cudaFree(x);
 }
@@ -892,18 +759,19 @@ static int build_paths(dp_ctx* ctx, const dp_grid& gr, const dp_ray* d_rays_in, 
   const dp_ray* rays = copy_rays ? P->rays : d_rays_in;
   P->row_ptr = static_cast<int64_t*>(perm_alloc(sizeof(int64_t) * (n_rays + 1)));
   P->geom = static_cast<float4*>(perm_alloc(sizeof(float4) * n_rays));
+  P->star = static_cast<double2*>(perm_alloc(sizeof(double2) * n_rays));
   int32_t* slot_cell = T.take<int32_t>(size_t(n_rays) * cap);
   double* slot_len = T.take<double>(size_t(n_rays) * cap);
   int64_t* counts = T.take<int64_t>(n_rays + 1);
   int64_t* totals = T.take<int64_t>(nbr + 2);
-  if (!P->row_ptr || !P->geom || !slot_cell || !slot_len || !counts || !totals)
+  if (!P->row_ptr || !P->geom || !P->star || !slot_cell || !slot_len || !counts || !totals)
     return bail(DP_ERR_ALLOC, "device allocation failed");
   GridDev g = grid_dev(gr);
   timed_begin(ctx);
   // 32 rays per block: the serial FP64 march spreads over all SMs
   trace_kernel<<<int((n_rays + 31) / 32), 32, 0, ctx->stream>>>(g, rays, n_rays, cap, side_cell,
                                                                      slot_cell, slot_len, counts,
-                                                                     P->geom, ctx->d_flag);
+                                                                     P->geom, P->star, ctx->d_flag);
   timed_end(ctx, "tomo_trace");
   launch_scan(ctx, counts, P->row_ptr, n_rays, totals);
   int64_t nnz = 0;
@@ -1009,6 +877,7 @@ static int make_eval(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
   P.side_density = tp->side_density;
   P.rays = pa->rays;
   P.geom = pa->geom;
+  P.star = pa->star;
   P.order = pa->order;
   P.n_rays = pa->n_rays;
   P.row_ptr = pa->row_ptr;
@@ -1040,8 +909,27 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
   P.nw = nw;
   P.flux = flux;
   const bool adj = (cot && grad) || jac || jraw;
-  // slot 1: node starts, then the Jacobian values
-  size_t need = size_t(P.n_nodes) * sizeof(NodeInit) + size_t(pa->nnz + 1) * 8 + 1024;
+  long blocks = std::min<long>((pa->n_rays + kWarps - 1) / kWarps, 152L * 16);
+  size_t smem = 0, work = 0;
+  int warps = kWarps;
+  if (precision == 0) {
+    // as many warps per CTA as the segment lists and tables leave room for, and
+    // no more CTAs than the device holds (each warp keeps its segments' terms)
+    int optin = 0, n_sm = 0, per_sm = 0;
+    DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+    const size_t most = size_t(optin) - 64;  // the kernel's own barrier
+    while (warps > 1 && eval64_smem(P.tab.ld, P.seg_cap, warps, adj) > most) warps /= 2;
+    smem = eval64_smem(P.tab.ld, P.seg_cap, warps, adj);
+    if (smem > most) return fail(ctx, DP_ERR_ARG, "ray too long for the FP64 kernel");
+    auto kernel = adj ? eval64_kernel<true> : eval64_kernel<false>;
+    DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
+    blocks = std::min<long>((pa->n_rays + warps - 1) / warps, long(std::max(per_sm, 1)) * n_sm);
+    if (adj) work = size_t(blocks) * warps * P.seg_cap * 32 * sizeof(double2);
+  }
+  // slot 1: node starts, then the Jacobian values and the FP64 adjoint's terms
+  size_t need = size_t(P.n_nodes) * sizeof(NodeInit) + size_t(pa->nnz + 1) * 8 + work + 2048;
   Arena A;
   A.base = static_cast<char*>(scratch(ctx, need, 1));
   A.cap = ctx->slot_bytes[1];
@@ -1053,23 +941,22 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
                                     : A.take<char>(size_t(pa->nnz + 1) * (precision ? 4 : 8));
     if (!jbuf) return fail(ctx, DP_ERR_ALLOC, "scratch allocation failed");
   }
-  long blocks = std::min<long>((pa->n_rays + kWarps - 1) / kWarps, 152L * 16);
-  size_t smem;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(eval64_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(eval64_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(eval32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(eval32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     attr = true;
   }
   timed_begin(ctx);
   if (precision == 0) {
-    smem = size_t(T_NCOL) * P.tab.ld * 8 + size_t(kWarps) * P.seg_cap * 3 * 8;
-    if (smem > 220 * 1024) return fail(ctx, DP_ERR_ARG, "ray too long for the FP64 kernel");
     P.jval64 = static_cast<double*>(jbuf);
-    if (adj) eval64_kernel<true><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
-    else eval64_kernel<false><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
+    if (adj) {
+      P.work = A.take<double2>(work / sizeof(double2));
+      if (!P.work) return fail(ctx, DP_ERR_ALLOC, "scratch allocation failed");
+      eval64_kernel<true><<<int(blocks), warps * 32, smem, ctx->stream>>>(P);
+    } else {
+      eval64_kernel<false><<<int(blocks), warps * 32, smem, ctx->stream>>>(P);
+    }
   } else {
     smem = size_t(2 * kNC32) * P.ld32 * 4 + size_t(kWarps) * P.seg_cap * 3 * 4 +
            size_t(P.n_nodes) * sizeof(NodeInit);
@@ -1206,7 +1093,7 @@ int host_eval(dp_ctx* ctx, const dp_physics* ph, const dp_grid* gr, const dp_tom
   const size_t cap = size_t(std::min(1001, gr->nx + gr->ny + gr->nz + 64) + 1);
   size_t bound = size_t(n_rays) * cap;  // segments cannot exceed this
   size_t need = size_t(n_rays) * cap * 12 + bound * (4 + 8 + 4 + 4 + 4 + 8) + size_t(ncell + 1) * 28 +
-                size_t(n_rays + 2) * (8 + 16 + 8 + 4) + size_t(ncell / kScan + n_rays / kScan + 8) * 16 +
+                size_t(n_rays + 2) * (8 + 16 + 16 + 8 + 4) + size_t(ncell / kScan + n_rays / kScan + 8) * 16 +
                 64 * 256;
   Arena A;
   A.base = static_cast<char*>(scratch(ctx, need, 3));
