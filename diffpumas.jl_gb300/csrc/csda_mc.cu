@@ -1,9 +1,10 @@
 // csda_mc.cu -- backward Monte Carlo in CSDA mode (run_backward_mc with
 // straggling = scattering = false) and its density derivative.
 //
-// One thread per history.  The history follows the adaptive two-layer step
-// sequence of src/Geometry.jl:534-672 (transport_backward_step :424-457,
-// step limit :461-476) and the acceptance of :694-757.  The derivative with
+// The history follows the adaptive two-layer step sequence of
+// src/Geometry.jl:534-672 (transport_backward_step :424-457, step limit
+// :461-476) and the acceptance of :694-757: FP64 in csda_fp64.cuh, one history
+// per warp or per thread; mixed precision below, one per thread.  The derivative with
 // respect to the rock density is propagated in tangent (forward) mode through
 // the same discrete program: for a single scalar density this is the cheapest
 // exact adjoint and equals what Zygote computes on the reference
@@ -17,6 +18,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fp64_math.cuh"
 #include "internal.h"
 
 namespace dp {
@@ -52,7 +54,7 @@ struct CsdaParams {
   double emin, emax;
   long n;
   const double *E, *q, *w;
-  double *contrib, *dcontrib, *sample_out;
+  double *contrib, *dcontrib;
   int32_t* steps;
   int* err_flag;  // 1: a table-staging wait gave up; 4: a history reached step_cap
   int step_cap, wait_iters;
@@ -63,191 +65,7 @@ struct CsdaParams {
   long n_los;
 };
 
-// Shared-memory table slots (all materials share the energy grid): the six
-// staged columns, then per-interval columns derived from them once per block
-// (1 / (R[i+1] - R[i]) and S[i+1] - S[i] per material, log-energy widths).
-enum { S_E = 0, S_LOGE, S_RS, S_RR, S_AS, S_AR, S_NCOL };
-enum { D_RINV = 0, D_RDS, D_AINV, D_ADS, D_DLE, D_NCOL };
-constexpr int kCsdaThreads = 64;
-
-// d(a^-1/2) = -1/2 a^-3/2 da
-__device__ __forceinline__ Dd drsqrt(Dd a) {
-  double r = rsqrt(a.v);
-  return Dd{r, -0.5 * r * r * r * a.d};
-}
-
-// One material's columns as one history walks them.
-struct CsdaMat {
-  const double *R, *S, *rinv, *ds;
-};
-
-// The CSDA history loop of run_backward_mc (src/Geometry.jl:534-672 with
-// transport_backward_step, :424-457, and the step limit, :461-476), in FP64
-// with the density tangent, arranged so that one step costs one exp and one
-// rsqrt:
-//  - the range at the end of a step is carried into the next step (the
-//    reference recomputes it from the energy: R(K(Y)) = Y to rounding);
-//  - the inverse range locates Y's interval and gives log E' = logE[i] +
-//    t dlogE[i] without a log, and S(E') = S[i] + t dS[i] on the same
-//    interval and parameter (the reference interpolates S at log(E'), the
-//    same point to rounding);
-//  - the stopping-power ratios S(E')/S(E) of consecutive steps in one
-//    material telescope to S(end)/S(start) of the material's run, and the
-//    decay factors multiply to exp(-sum dt / c tau);
-//  - beta gamma = sqrt(gamma^2 - 1) with gamma the mean of the step's end
-//    points, so dt = step * rsqrt(gamma^2 - 1).
-// Every branch the reference takes (boundaries, step limits and clamps, the
-// energy ceiling, the acceptance) is the same, and the results agree with
-// the reference's operation-by-operation program to rounding (~1e-13).
-__global__ void __launch_bounds__(kCsdaThreads) csda_mc_kernel(CsdaParams P) {
-  extern __shared__ __align__(16) double smem[];
-  __shared__ uint64_t mbar;
-  const int ld = P.tab.ld, n = P.tab.n;
-  const double* src[S_NCOL] = {P.tab.col(0, DP_COL_E),          P.tab.col(0, DP_COL_LOGE),
-                               P.tab.col(P.rock, DP_COL_CSDA_S), P.tab.col(P.rock, DP_COL_CSDA_R),
-                               P.tab.col(P.air, DP_COL_CSDA_S),  P.tab.col(P.air, DP_COL_CSDA_R)};
-  if (!stage_columns(smem, src, S_NCOL, uint32_t(ld * sizeof(double)), &mbar, P.wait_iters)) {
-    if (threadIdx.x == 0) atomicExch(P.err_flag, 1);
-    return;
-  }
-  const double* sE = smem + S_E * ld;
-  const double* slE = smem + S_LOGE * ld;
-  double* der = smem + S_NCOL * ld;
-  for (int k = threadIdx.x; k < n - 1; k += blockDim.x) {
-    const double* rR = smem + S_RR * ld;
-    const double* rS = smem + S_RS * ld;
-    const double* aR = smem + S_AR * ld;
-    const double* aS = smem + S_AS * ld;
-    der[D_RINV * ld + k] = 1.0 / (rR[k + 1] - rR[k]);
-    der[D_RDS * ld + k] = rS[k + 1] - rS[k];
-    der[D_AINV * ld + k] = 1.0 / (aR[k + 1] - aR[k]);
-    der[D_ADS * ld + k] = aS[k + 1] - aS[k];
-    der[D_DLE * ld + k] = slE[k + 1] - slE[k];
-  }
-  __syncthreads();
-  const CsdaMat rockM{smem + S_RR * ld, smem + S_RS * ld, der + D_RINV * ld, der + D_RDS * ld};
-  const CsdaMat airM{smem + S_AR * ld, smem + S_AS * ld, der + D_AINV * ld, der + D_ADS * ld};
-  const double* dle = der + D_DLE * ld;
-  const double eps = kEps64;
-  const double half_inv_m = 0.5 / P.mass;
-  const int32_t cap = P.step_cap;
-  for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < P.n;
-       i += long(gridDim.x) * blockDim.x) {
-    double E0, q, w;
-    CsdaGeo G = P.geo;
-    if (P.los) {
-      long lo = 0, hi = P.n_los;
-      while (hi - lo > 1) {
-        long mid = (lo + hi) >> 1;
-        if (P.los_off[mid] <= i) lo = mid; else hi = mid;
-      }
-      const dp_los& L = P.los[lo];
-      double H = L.air_height > 0.0 ? L.thickness + L.air_height
-                                    : (L.primary_altitude > 0.0 ? L.primary_altitude : 3e4);
-      G = csda_geo(L.thickness, L.density, L.elevation, H);
-      mc_sample(P.seed, uint64_t(i), L.energy_min,
-                L.energy_max > L.energy_min ? L.energy_max : L.energy_min, &E0, &q, &w);
-    } else if (P.use_philox) {
-      mc_sample(P.seed, uint64_t(i), P.emin, P.emax, &E0, &q, &w);
-      if (P.sample_out) {
-        P.sample_out[3 * i] = E0;
-        P.sample_out[3 * i + 1] = q;
-        P.sample_out[3 * i + 2] = w;
-      }
-    } else {
-      E0 = P.E[i];
-      q = P.q[i];
-      w = P.w[i];
-    }
-    const Dd rho = dd(G.rho, 1.0);
-    const Dd c_rock = dd(0.01, 0.0) / dmax(rho, dd(1e-6));  // 0.01 / rho
-    const double inv_uz = G.uz > eps || G.uz < -eps ? 1.0 / G.uz : 0.0;
-    Dd E = dd(E0), lE = dd(log(E0)), z = dd(0.0), tau = dd(0.0);
-    Dd wS = dd(1.0), Sstart = dd(1.0), Scur = dd(1.0), X = dd(0.0);
-    int mat = -1, k = 0;
-    int32_t nsteps = 0;
-    while (nsteps < cap) {
-      if (!(E.v < P.threshold - eps)) break;
-      if (z.v < 0.0 || z.v >= G.H - eps) break;
-      const int m = z.v >= G.thickness ? 1 : 0;
-      const CsdaMat M = m ? airM : rockM;
-      if (m != mat) {
-        // entering a material: range and stopping power at E from the
-        // log-energy interpolation (src/Physics.jl:660-687), as the
-        // reference's first step in it does
-        if (mat >= 0) wS = wS * (Scur / Sstart);
-        mat = m;
-        X = interp_logE(P.tab, sE, slE, M.R, E, lE, nullptr);
-        Sstart = interp_logE(P.tab, sE, slE, M.S, E, lE, nullptr);
-        Scur = Sstart;
-        k = E.v <= sE[0] ? 0 : (E.v >= sE[n - 1] ? n - 2
-                                                  : uniform_interval(slE, n, lE.v, P.tab.lE0,
-                                                                     P.tab.inv_dlE));
-      }
-      Dd dens, tob, lim;
-      if (m == 0) {
-        dens = rho;
-        if (G.uz > eps) tob = (dd(G.thickness) - z) * inv_uz;
-        else if (G.uz < -eps) tob = (dd(0.0) - z) * inv_uz;
-        else tob = dd(1000.0);
-        lim = X * c_rock;
-      } else {
-        dens = 1.205 * dexp(z / -12e3);
-        if (G.uz > eps) tob = (dd(G.H) - z) * inv_uz;
-        else if (G.uz < -eps) tob = (dd(G.thickness) - z) * inv_uz;
-        else tob = dd(1000.0);
-        lim = dmin(0.01 * X / dmax(dens, dd(1e-6)), dd(G.air_limit));
-      }
-      Dd step = dmin(tob + dd(1e-7), lim);
-      if (step.v < kStepMin) step = dd(kStepMin);
-      else if (step.v > 1000.0) step = dd(1000.0);
-      // inverse range at Y (src/Physics.jl:833-867), clamped at the table ends
-      const Dd Y = X + step * dens;
-      Dd Ef, lEf, Sf;
-      if (Y.v <= M.R[0]) {
-        k = 0;
-        Ef = dd(sE[0]);
-        lEf = dd(slE[0]);
-        Sf = dd(M.S[0]);
-      } else if (Y.v >= M.R[n - 1]) {
-        k = n - 2;
-        Ef = dd(sE[n - 1]);
-        lEf = dd(slE[n - 1]);
-        Sf = dd(M.S[n - 1]);
-      } else {
-        k = walk_up(M.R, n, Y.v, k);
-        const Dd t = (Y - dd(M.R[k])) * M.rinv[k];
-        lEf = dd(slE[k]) + t * dle[k];
-        Ef = dexp(lEf);
-        Sf = dd(M.S[k]) + t * M.ds[k];
-      }
-      // proper time of the step at the mean Lorentz factor
-      const Dd ga = dd(1.0) + (E + Ef) * half_inv_m;
-      const Dd g2 = ga * ga - dd(1.0);
-      const Dd dt = g2.v > 1e-12 * ga.v * ga.v ? step * drsqrt(g2) : step / (1e-6 * ga);
-      tau = tau + dt;
-      z = z - step * dd(G.dir_z);
-      X = Y;
-      E = Ef;
-      lE = lEf;
-      Scur = Sf;
-      ++nsteps;
-    }
-    if (mat >= 0) wS = wS * (Scur / Sstart);
-    const Dd wt = wS * dexp(tau / -P.ctau);
-    double f = 0.0, df = 0.0;
-    if (nsteps >= cap) atomicExch(P.err_flag, 4);
-    else if (z.v >= G.H - 1.0 && E.v < P.threshold && G.cos_final > 0.0) {
-      double dlogf;
-      double F = gccly_flux(G.cs, G.cs129, E.v, q, &dlogf);
-      f = wt.v * F;
-      df = wt.d * F + wt.v * F * dlogf * E.d;
-    }
-    P.contrib[i] = w * f;
-    if (P.dcontrib) P.dcontrib[i] = w * df;
-    if (P.steps) P.steps[i] = nsteps;
-  }
-}
+#include "csda_fp64.cuh"
 
 // ------------------------------------------------------------ mixed precision
 // The same history loop with the transport and its density tangent in FP32
@@ -307,7 +125,7 @@ __device__ __forceinline__ int f_interval(const Tab32& t, int n, float lx, const
   return i;
 }
 
-// The lean step of csda_mc_kernel in FP32: one exponential and one rsqrt per
+// The lean step of the FP64 kernels in FP32: one exponential and one rsqrt per
 // step, telescoped stopping-power ratios, a summed decay exponent.  What
 // keeps a history within ~1e-6 of the FP64 program:
 //  - the range and its density tangent are float pairs (TwoSum), so that
@@ -652,9 +470,26 @@ static int setup(dp_ctx* ctx, const dp_physics* ph, const dp_mc_params* p, CsdaP
   return DP_OK;
 }
 
-// One wave of resident blocks whose threads stride over the histories (a
-// grid of several partial waves idles SMs at its end).
+// Whether the FP64 histories go one to a warp.  Both forms issue about as many
+// instructions per history where the warp's batches are closed forms: in the
+// rock, and in the air once the step is the altitude limit, that is above the
+// range X = 100 air_limit 1.205 kg/m^2.  Behind at least that much rock the warp
+// form is the faster one at any number (45 deg, 100 m, 10^4 histories: 0.78
+// against 1.70 ms by thread; 10^5: 6.0 against 8.3).  Behind less, the steps of
+// 1 % in the air chain over the altitude, and it is faster only while the
+// threads leave the chip idle (70 deg, 5 m, 1-20 GeV: 10^3 histories 0.23
+// against 0.80 ms, 10^4 1.24 against 0.83, 10^5 9.9 against 3.9).  Lines of
+// sight of a batch differ, so they follow the second rule.
+static bool csda_by_warp(const CsdaParams& P) {
+  const double grammage = P.geo.thickness * P.geo.rho / std::fmax(std::fabs(P.geo.uz), 0.05);
+  const bool thick = !P.los && grammage >= 100.0 * P.geo.air_limit * 1.205;
+  return thick || P.n <= 5000;
+}
+
+// One wave of resident blocks whose warps or threads stride over the histories
+// (a grid of several partial waves idles SMs at its end).
 static int launch(dp_ctx* ctx, CsdaParams& P, const dp_physics* ph32 = nullptr) {
+  const bool by_warp = !ph32 && csda_by_warp(P);
   const int threads = ph32 ? 128 : kCsdaThreads;
   const size_t smem = ph32 ? size_t(2 * F_NCOL) * ph32->ld32 * sizeof(float)
                            : size_t(S_NCOL + D_NCOL) * P.tab.ld * sizeof(double);
@@ -662,18 +497,26 @@ static int launch(dp_ctx* ctx, CsdaParams& P, const dp_physics* ph32 = nullptr) 
   if (ph32)
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csda32_kernel, threads,
                                                                      smem));
-  else
-    DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csda_mc_kernel,
+  else if (!by_warp)
+    DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csda_thread_kernel,
                                                                      threads, smem));
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
+  // by warp: two warps per SM partition (the second covers the first's waits),
+  // each with a group of histories so that a warp evaluates their fluxes together
+  const long warps = long(n_sm) * 2 * (threads / 32);
+  const long rounds = std::max<long>(1, (P.n + 32 * warps - 1) / (32 * warps));
+  const int group = int(std::max<long>(1, (P.n + rounds * warps - 1) / (rounds * warps)));
   long blocks = (P.n + threads - 1) / threads;
-  blocks = std::min(blocks, long(std::max(per_sm, 1)) * n_sm);
+  if (by_warp) blocks = std::min((P.n + group - 1) / group, long(n_sm) * 2);
+  else blocks = std::min(blocks, long(std::max(per_sm, 1)) * n_sm);
   if (blocks < 1) blocks = 1;
   timed_begin(ctx);
   if (ph32)
     csda32_kernel<<<int(blocks), threads, smem, ctx->stream>>>(P, ph32->dev32, ph32->ld32);
+  else if (by_warp)
+    csda_warp_kernel<<<int(blocks), threads, smem, ctx->stream>>>(P, group);
   else
-    csda_mc_kernel<<<int(blocks), threads, smem, ctx->stream>>>(P);
+    csda_thread_kernel<<<int(blocks), threads, smem, ctx->stream>>>(P);
   DP_CHECK_CUDA(ctx, cudaGetLastError());
   timed_end(ctx, ph32 ? "csda_mc32" : "csda_mc");
   return DP_OK;

@@ -109,5 +109,19 @@ __device__ __forceinline__ double uniform(uint32_t a, uint32_t b) {
   return __longlong_as_double((m << (z - 11) & 0xfffffffffffffull) | (uint64_t(1033 - z) << 52));
 }
 
+// 1 / (beta gamma) at the kinetic energy x (in masses), beta >= 1e-6, and its
+// derivative in x (src/Geometry.jl:1083-1107).
+__device__ __forceinline__ double inv_beta_gamma(double x, double* d) {
+  if (hi32(x) < 0x3d719799) {  // x < 1e-12: the clamp of beta
+    const double g = 1.0 + x, b2 = 1.0 - 1.0 / (g * g);
+    const double b = ::sqrt(b2 >= 1e-12 ? b2 : 1e-12), r = 1.0 / (b * g);
+    *d = b2 >= 1e-12 ? -r / (b2 * g * g * g) - r / g : -r / g;
+    return r;
+  }
+  const double r = rsqrt(x * (x + 2.0));  // gamma^2 - 1
+  *d = -(x + 1.0) * (r * r * r);
+  return r;
+}
+
 }  // namespace f64
 }  // namespace dp

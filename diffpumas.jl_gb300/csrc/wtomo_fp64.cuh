@@ -148,20 +148,6 @@ __device__ __forceinline__ void begin(const Tables& tb, const M& m, Walk<N>& k) 
 __device__ __forceinline__ bool positive_finite(double x) {
   return uint32_t(f64::hi32(x) - 1) < 0x7fefffffu;
 }
-// 1 / (beta gamma) at the kinetic energy x (in masses), beta >= 1e-6, and its
-// derivative in x (src/Geometry.jl:1083-1107).
-__device__ __forceinline__ double inv_bg(double x, double* d) {
-  const double y = x * (x + 2.0);  // gamma^2 - 1
-  if (f64::hi32(x) < 0x3d719799) {  // x < 1e-12: the clamp of beta
-    const double g = 1.0 + x, b2 = 1.0 - 1.0 / (g * g);
-    const double b = ::sqrt(b2 >= 1e-12 ? b2 : 1e-12), r = 1.0 / (b * g);
-    *d = b2 >= 1e-12 ? -r / (b2 * g * g * g) - r / g : -r / g;
-    return r;
-  }
-  const double r = f64::rsqrt(y);
-  *d = -(x + 1.0) * (r * r * r);
-  return r;
-}
 // One Heun step of length ds and grammage gx (src/Tomography.jl:455-471) from
 // k to k; false on an invalid step (k is then not to be kept).
 template <int N, class M>
@@ -177,7 +163,7 @@ __device__ __forceinline__ bool heun(const Tables& tb, const Run& R, const M& m,
   const Val v2 = m.at(p2);
   const double iEn = f64::rcp(En), a2 = v2.sl * iEn;
   double dib;
-  const double x = (k.E + En) * R.half_inv_m, ib = inv_bg(x, &dib);
+  const double x = (k.E + En) * R.half_inv_m, ib = f64::inv_beta_gamma(x, &dib);
 #pragma unroll
   for (int n = 0; n < N; ++n) {
     const double dEp = fma(k.S, dgx[n], fma(k.dS[n], gx, k.dE[n]));
