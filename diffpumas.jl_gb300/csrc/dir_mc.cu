@@ -324,18 +324,32 @@ struct PathGeo {
     const Med<R>& m = meds[h.med];
     const bool air = h.stage == 2;
     // locals_air_at_altitude (src/Geometry.jl:95-106) at detector elevation + z
-    const R rho = air ? R(1.205) * exp(-(R(P.B.detector_elevation) + alt_r(s.z)) / R(12e3)) : h.rho;
-    const Loc<R> Li = locate(m, s.E);
-    R mx = R(0.01) * at(m, Li, MC_CR) / fmax(rho, air ? R(1e-8) : R(1e-6));
-    if (air) mx = fmin(mx, R(0.05 * 12e3) / fmax(h.cos_t, R(0.05)));
+    R rho, mx, lE = R(0);  // FP64: the logarithm of the energy serves the whole step
+    Loc<R> Li;
+    if constexpr (sizeof(R) == 8) {
+      rho = air ? 1.205 * f64::exp((P.B.detector_elevation + s.z) * (-1.0 / 12e3)) : h.rho;
+      lE = f64::log(s.E);
+      Li = locate_log(m, s.E, lE);
+      mx = f64::div(0.01 * at(m, Li, MC_CR), f64::max_pos(rho, air ? 1e-8 : 1e-6));
+      if (air) mx = f64::min_pos(mx, f64::div(0.05 * 12e3, f64::max_pos(h.cos_t, 0.05)));
+    } else {
+      rho = air ? R(1.205) * exp(-(R(P.B.detector_elevation) + alt_r(s.z)) / R(12e3)) : h.rho;
+      Li = locate(m, s.E);
+      mx = R(0.01) * at(m, Li, MC_CR) / fmax(rho, air ? R(1e-8) : R(1e-6));
+      if (air) mx = fmin(mx, R(0.05 * 12e3) / fmax(h.cos_t, R(0.05)));
+    }
     const R step = fmin(h.remaining, fmax(R(1e-6), fmin(h.remaining + R(1e-7), mx)));
     h.d0 = h.dist;
     h.E0 = s.E;
     h.limit = limit;
     if (C.straggling) {
       if constexpr (PHASE == 0) {
-        if (straggled_step<R, true, true>(m, C, s, Li, R(0), rho, step, g, false, limit,
-                                                h.x)) {
+        bool waits;
+        if constexpr (sizeof(R) == 8)
+          waits = straggled_step64<true>(m, C, s, Li, lE, 0.0, rho, step, g, false, limit, h.x);
+        else
+          waits = straggled_step<R, true, true>(m, C, s, Li, R(0), rho, step, g, false, limit, h.x);
+        if (waits) {
           h.x.kind = CONT_STRAG;
           h.x.medium = h.med;
           return ADV_WAIT;
@@ -366,7 +380,7 @@ struct PathGeo {
         mixed_end(h.s, x, Emax, h.limit, false);
       } else {
         ++x.event;
-        if (mixed_run_in<R>(m, P.C, h.s, x, g, h.limit)) {
+        if (mixed_again(m, P.C, h.s, x, g, h.limit)) {
           x.kind = CONT_MIXED;
           return ADV_WAIT;
         }

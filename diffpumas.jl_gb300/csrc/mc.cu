@@ -224,8 +224,10 @@ Layout make_layout(const dp_mixture* const* media, int n_media, size_t esize) {
   int nel = 0;
   for (int k = 0; k < n_media; ++k) nel = std::max(nel, media[k]->nel);
   L.o_phys = uint32_t((kEldOffset + (esize == 8 ? nel * kEldStride : 0)) * sizeof(double));
-  L.o_ker = L.o_phys + uint32_t(size_t(MC_LB1 + 2 * L.slots) * L.ld * esize);
-  L.o_idx = L.o_ker + uint32_t(size_t(K_NCOL) * L.ldk * esize);
+  // FP64 media carry the inverse interval widths too (pack_derived)
+  const int dp = esize == 8 ? X_NCOL : 0, dk = esize == 8 ? 1 : 0;
+  L.o_ker = L.o_phys + uint32_t(size_t(MC_LB1 + 2 * L.slots + dp) * L.ld * esize);
+  L.o_idx = L.o_ker + uint32_t(size_t(K_NCOL + dk) * L.ldk * esize);
   L.nbp = kIdxBinsPhys;
   L.nbk = kIdxBinsKer;
   uint32_t idx_bytes = uint32_t((2 * kIdxBinsPhys + 2 * kIdxBinsKer) * sizeof(int16_t));
@@ -271,6 +273,17 @@ static void pack_dcs(const dp_mixture* m, double* out) {
   }
 }
 
+// The derived columns of an FP64 medium: inverse interval widths.
+static void pack_derived(const dp_mixture* m, const Layout& L, double* P, double* K) {
+  auto inv = [](double* dst, const double* y, int n) {
+    for (int i = 0; i + 1 < n; ++i) dst[i] = y[i + 1] != y[i] ? 1.0 / (y[i + 1] - y[i]) : 0.0;
+  };
+  const int src[X_NCOL] = {MC_LE, MC_CR, MC_MR};
+  for (int k = 0; k < X_NCOL; ++k)
+    inv(P + size_t(MC_LB1 + 2 * L.slots + k) * L.ld, P + size_t(src[k]) * L.ld, m->n);
+  inv(K + size_t(K_IE) * L.ldk, K + size_t(K_E) * L.ldk, m->nk);
+}
+
 template <class R>
 static void pack(const dp_mixture* m, const Layout& L, unsigned char* out) {
   std::memset(out, 0, L.med_bytes);
@@ -299,7 +312,10 @@ static void pack(const dp_mixture* m, const Layout& L, unsigned char* out) {
     f[4] = float(kAvogadro / (x[1] * 0.001));
     f[5] = float(x[4]);  // nuclear RMS radius (DEL polar angles)
   }
-  if (sizeof(R) == 8) pack_dcs(m, reinterpret_cast<double*>(out) + kEldOffset);
+  if constexpr (sizeof(R) == 8) {
+    pack_dcs(m, reinterpret_cast<double*>(out) + kEldOffset);
+    pack_derived(m, L, P, K);
+  }
   // index tables of the inverse lookups (origins and widths in R)
   R* prm = reinterpret_cast<R*>(reinterpret_cast<double*>(out) + kMaxEl * kElStride);
   int16_t* idx = reinterpret_cast<int16_t*>(out + L.o_idx);

@@ -1,7 +1,7 @@
 // mc_device.cuh -- device side of the stochastic backward Monte Carlo: one
 // thread per history, templated on the transport arithmetic R (double: the
-// reference's FP64 operations; float: the mixed-precision form, where
-// positions, event kinematics, DCS and the flux stay FP64).
+// FP64 transport, whose steps are in mc_fp64.cuh; float: the mixed-precision
+// form, where positions, event kinematics, DCS and the flux stay FP64).
 //
 // Restates src/Geometry.jl:148-357 (straggled step), :424-457 (CSDA step),
 // :461-476 (step limit), :534-672 (dual-mode loop), :694-757 (acceptance),
@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "dcs.cuh"
+#include "fp64_math.cuh"
 
 namespace dp {
 namespace mc {
@@ -168,6 +169,12 @@ struct Consts {
   }
 };
 
+// log and exp of the FP64 transport, out of line: a step calls some twenty of
+// them, and inlined they push the step out of the instruction cache (10^4
+// histories of run_backward_mc 29.6 -> 27.3 ms, 10^5 117.6 -> 107.9 ms).
+static __device__ __noinline__ double log64(double x) { return f64::log(x); }
+static __device__ __noinline__ double exp64(double x) { return f64::exp(x); }
+
 // ------------------------------------------------------------ random stream
 struct Stream {
   uint32_t k0, k1, c0, c1, block, w0, w1, w2, w3;
@@ -206,7 +213,7 @@ template <class R> __device__ __forceinline__ R uni(Stream& g);
 template <> __device__ __forceinline__ double uni<double>(Stream& g) {
   uint32_t a, b;
   g.next(a, b);
-  return u01(a, b);
+  return f64::uniform(a, b);
 }
 // The leading 24 bits of the same draw (it differs from the double by < 2^-24).
 // FP32: 24 bits of the draw, in (0, 1).  A 24-bit uniform of exactly 0
@@ -224,6 +231,10 @@ __device__ __forceinline__ double uni_d(Stream& g) {
   return u01(a, b);
 }
 template <class R> __device__ __forceinline__ R expo(Stream& g) { return -log1p(-uni<R>(g)); }
+// 1 - u is exact: u is a multiple of 2^-53
+template <> __device__ __forceinline__ double expo<double>(Stream& g) {
+  return -log64(1.0 - uni<double>(g));
+}
 
 template <class R> __device__ __forceinline__ R ulp_up(R x);
 template <> __device__ __forceinline__ double ulp_up<double>(double x) {
@@ -575,7 +586,8 @@ static __device__ __noinline__ void coop_batch(const float* elf, int nel, float 
 // (standard rock: 21 points instead of 168, with the element's own powers of Z
 // and A packed once per medium).  run_backward_mc of 10^4 histories through
 // 100 m of rock: 1330 -> 78.5 ms with full warps; 2 10^4 histories through the
-// rock/water/air mixture 3.2 s -> 0.1 s.
+// rock/water/air mixture 3.2 s -> 0.1 s; with the functions of fp64_math.cuh in
+// the terms 10^4 histories 27.3 -> 22.1 ms, 10^5 107.9 -> 72.6 ms.
 //
 // Per-warp buffer (doubles): 12 pair points of kPairPt, 9 photonuclear points
 // of kPhotoPt, then per element the pair prefactor, 4 components and 12 items.
@@ -603,11 +615,11 @@ __device__ __forceinline__ void del64_pair_point(double mass, double K, double q
                                                  double* o) {
   const double me = kMeMeV;
   const double energy = (K + mass) * 1e3, v = q / (K + mass), m = mass * 1e3;
-  const double r = exp(gl12(i, false) * tmin), rho = 1.0 - r, r2 = rho * rho;
-  const double iv1 = 1.0 / (1.0 - v), beta = 0.5 * v * v * iv1;
+  const double r = exp64(gl12(i, false) * tmin), rho = 1.0 - r, r2 = rho * rho;
+  const double iv1 = f64::rcp(1.0 - v), beta = 0.5 * v * v * iv1;
   const double h = m * v / (2.0 * me), xi = h * h * (1.0 - r2) * iv1;
-  const double ixi = 1.0 / xi, op = 1.0 + xi, iop = 1.0 / op;
-  const double lxi = log(1.0 + ixi), l1x = log(op);
+  const double ixi = 1.0 / xi, op = 1.0 + xi, iop = f64::rcp(op);
+  const double lxi = log64(1.0 + ixi), l1x = log64(op);
   // Li2 of a = 1/(1 + xi) and of b = 1 - a: the series at the smaller of the
   // two, the other by reflection (log b = -lxi, log a = -l1x)
   const bool lo = iop <= 0.5;
@@ -619,8 +631,8 @@ __device__ __forceinline__ void del64_pair_point(double mass, double K, double q
   const double Ce2 = ((1.0 - r2) * (1.0 + beta) + xi * (3.0 - r2)) * lxi +
                      2.0 * (1.0 - beta - r2) * iop - (3.0 - r2);
   const double De = ae * dl1 - (2.0 + r2) * xi * lxi - (xi + r2 + beta) * iop;
-  const double t = De / Be;
-  const double Xe = fabs(t) < 100.0 ? exp(-fabs(t)) : 0.0;
+  const double t = f64::div(De, Be);
+  const double Xe = fabs(t) < 100.0 ? exp64(-fabs(t)) : 0.0;
   const double b2 = 1.0 + 2.0 * beta;
   const double bb = (1.0 + r2) * (1.0 + 1.5 * beta) - ixi * b2 * (1.0 - r2);
   const double Bm = bb * l1x + xi * (1.0 - r2 - beta) * iop + b2 * (1.0 - r2);
@@ -628,12 +640,12 @@ __device__ __forceinline__ void del64_pair_point(double mass, double K, double q
                      2.0 * (1.0 - beta - r2) * iop + 1.0 - beta - (1.0 + beta) * r2;
   const double Dm = bb * dl2 + (1.0 + 1.5 * beta) * (1.0 - r2) * ixi * l1x +
                     (1.0 - r2 - 0.5 * beta * (1.0 + r2) + (1.0 - r2) * 0.5 * ixi * beta) * xi * iop;
-  const double s = Dm / Bm;
-  const double Xm = fabs(s) < 100.0 ? exp(-fabs(s)) : 0.0;
+  const double s = f64::div(Dm, Bm);
+  const double Xm = fabs(s) < 100.0 ? exp64(-fabs(s)) : 0.0;
   o[0] = Be - Ce2;
   o[1] = Ce2;
-  o[2] = sqrt(op);
-  o[3] = 2.0 * me * op / (energy * v * (1.0 - r2));
+  o[2] = f64::sqrt(op);
+  o[3] = f64::div(2.0 * me * op, energy * v * (1.0 - r2));
   o[4] = op;
   // t > 0: log(. / (X + .)) - t ..., t <= 0: log(. / (1 + X .)) - t/2 ...
   o[5] = t > 0.0 ? Xe : 1.0;
@@ -644,7 +656,7 @@ __device__ __forceinline__ void del64_pair_point(double mass, double K, double q
   o[10] = s > 0.0 ? Xm : 1.0;
   o[11] = s > 0.0 ? 1.0 : Xm;
   o[12] = s > 0.0 ? s : 0.0;
-  o[13] = -(r * gl12(i, true) * tmin) * 0.1 / energy;
+  o[13] = -(r * gl12(i, true) * tmin) * f64::div(0.1, energy);
 }
 // The point's term for one element (prefactor pre = cpf (Z + zeta)(1 - v)/v).
 __device__ __forceinline__ double del64_pair_item(const double* o, const double* el, double pre,
@@ -653,10 +665,10 @@ __device__ __forceinline__ double del64_pair_item(const double* o, const double*
   const double g1 = 0.8464817248906141, g2 = 0.7165313105737893;      // e^(-1/6), e^(-1/3)
   const double rlz = el[EL_RLZ], d = o[3] * rlz, y = o[4] * el[EL_MDN2];
   const double num = rlz * o[2];
-  const double Le1 = log(num / ((o[5] + o[6] * c1 * d) * sqrt(o[5] + o[6] * y))) - o[7];
-  const double Le2 = log(num * g1 / ((o[5] + o[6] * c2 * d) * sqrt(o[5] + o[6] * y * g2))) - o[7];
-  const double Lm1 = log(el[EL_PRE] / (o[10] + o[11] * c1 * d)) - o[12];
-  const double Lm2 = log(el[EL_PRE] / (o[10] + o[11] * c2 * d)) - o[12];
+  const double Le1 = log64(f64::div(num, (o[5] + o[6] * c1 * d) * f64::sqrt(o[5] + o[6] * y))) - o[7];
+  const double Le2 = log64(f64::div(num * g1, (o[5] + o[6] * c2 * d) * f64::sqrt(o[5] + o[6] * y * g2))) - o[7];
+  const double Lm1 = log64(f64::div(el[EL_PRE], o[10] + o[11] * c1 * d)) - o[12];
+  const double Lm2 = log64(f64::div(el[EL_PRE], o[10] + o[11] * c2 * d)) - o[12];
   const double de = pre * (o[0] * Le1 + o[1] * Le2);
   const double dm = pre * me_m2 * (o[8] * Lm1 + o[9] * Lm2);
   return ((de < 0.0 ? 0.0 : de) + (dm < 0.0 ? 0.0 : dm)) * o[13];
@@ -666,29 +678,29 @@ __device__ __forceinline__ double del64_pair_item(const double* o, const double*
 // shadowing exponent (positive: the constant low-x form, 0: none).
 __device__ __forceinline__ void del64_photo_point(double ml, double K, double q, double lmin, double dx,
                                                   int i, double* o) {
-  const double Q2 = exp(lmin + dx * gl9(i, false));
+  const double Q2 = exp64(lmin + dx * gl9(i, false));
   const double M = 0.5 * (kProtonMass + kNeutronMass), M2 = M * M, E = K + ml, y = q / E;
   const double x = 0.5 * Q2 / (M * q);
   const double m02 = 0.31985, mP2 = 49.457, mR2 = 0.15052, Q02 = 0.52544, L2 = 0.06527;
   const double W = M2 + Q2 * (1.0 / x - 1.0) - M2;
-  // t = log(log((Q2 + Q02) / L2) / log(Q02 / L2)); t^c = exp(c log t)
-  const double lt = log(log(log((Q2 + Q02) / L2) / 2.0857034941768826));
-  const double lxP = log((Q2 + mP2) / (Q2 + mP2 + W)), lxR = log((Q2 + mR2) / (Q2 + mR2 + W));
-  const double l1x = log(1.0 - x);
-  const double cP = 0.28067 + (0.28067 - 0.22291) * (1.0 / (1.0 + exp(2.1979 * lt)) - 1.0);
-  const double aP = -0.0808 + (-0.0808 + 0.44812) * (1.0 / (1.0 + exp(1.1709 * lt)) - 1.0);
-  const double bP = 0.36292 + 1.8917 * exp(1.8439 * lt);
-  const double cR = 0.80107 + 0.97307 * exp(3.4942 * lt);
-  const double aR = 0.58400 + 0.37888 * exp(2.6063 * lt);
-  const double bR = 0.01147 + 3.7582 * exp(0.49338 * lt);
-  const double F2 = Q2 / (Q2 + m02) * (cP * exp(aP * lxP + bP * l1x) + cR * exp(aR * lxR + bR * l1x));
+  // t = log(log((Q2 + Q02) / L2) / log(Q02 / L2)); t^c = exp64(c log t)
+  const double lt = log64(log64(log64((Q2 + Q02) / L2) / 2.0857034941768826));
+  const double lxP = log64(f64::div(Q2 + mP2, Q2 + mP2 + W)), lxR = log64(f64::div(Q2 + mR2, Q2 + mR2 + W));
+  const double l1x = log64(1.0 - x);
+  const double cP = 0.28067 + (0.28067 - 0.22291) * (f64::rcp(1.0 + exp64(2.1979 * lt)) - 1.0);
+  const double aP = -0.0808 + (-0.0808 + 0.44812) * (f64::rcp(1.0 + exp64(1.1709 * lt)) - 1.0);
+  const double bP = 0.36292 + 1.8917 * exp64(1.8439 * lt);
+  const double cR = 0.80107 + 0.97307 * exp64(3.4942 * lt);
+  const double aR = 0.58400 + 0.37888 * exp64(2.6063 * lt);
+  const double bR = 0.01147 + 3.7582 * exp64(0.49338 * lt);
+  const double F2 = Q2 / (Q2 + m02) * (cP * exp64(aP * lxP + bP * l1x) + cR * exp64(aR * lxR + bR * l1x));
   const double iE2 = 1.0 / (E * E);
   const double dds = (1.0 - y + 0.5 * (1.0 - 2.0 * ml * ml / Q2) * (y * y + Q2 * iE2)) / (Q2 * Q2) -
                      0.25 * iE2 / Q2;
   const double cf = 4.0 * kPi * kAlpha * kAlpha * kHbarC * kHbarC;
   o[0] = cf * F2 * dds / q * (gl9(i, true) * dx * Q2);
   o[1] = 1.0 + x * (-1.85 + x * (2.45 + x * (-2.35 + x)));
-  o[2] = x < 0.0014 ? -0.1 : (x < 0.04 ? 0.069 * log10(x) + 0.097 : 0.0);
+  o[2] = x < 0.0014 ? -0.1 : (x < 0.04 ? 0.069 * 0.4342944819032518 * log64(x) + 0.097 : 0.0);
 }
 // Bremsstrahlung of one element (src/Materials.jl:631-695), per mass.
 __device__ __forceinline__ double del64_brems(const double* el, double m, double K, double q) {
@@ -697,11 +709,11 @@ __device__ __forceinline__ double del64_brems(const double* el, double m, double
   const double energy = (K + m) * 1e3, v = q * 1e3 / energy, mm = m * 1e3;
   const double delta = mm * mm * v / (2.0 * energy * (1.0 - v)), rlz = el[EL_RLZ];
   const double e12 = 1.6487212707001282, e13 = 1.3956124250860895, em16 = 0.8464817248906141;
-  const double phi1 = log(rlz * (mm / me) / (1.0 + rlz * e12 * delta / me)) - el[EL_D1];
-  const double phi2 = log(rlz * em16 * (mm / me) / (1.0 + rlz * e13 * delta / me)) - el[EL_D2];
+  const double phi1 = log64(f64::div(rlz * (mm / me), 1.0 + rlz * e12 * delta / me)) - el[EL_D1];
+  const double phi2 = log64(f64::div(rlz * em16 * (mm / me), 1.0 + rlz * e13 * delta / me)) - el[EL_D2];
   const double sa = (4.0 / 3.0 * (1.0 - v) + v * v) *
-                    (log(mm / delta / (mm * delta / (me * me) + kSqrtE)) -
-                     log(1.0 + me / (delta * el[EL_RLI])));
+                    (log64(f64::div(mm, delta * (mm * delta / (me * me) + kSqrtE))) -
+                     log64(1.0 + f64::div(me, delta * el[EL_RLI])));
   double sr;
   if (v < 0.0 || v > 1.0) {
     sr = 0.0;
@@ -710,7 +722,7 @@ __device__ __forceinline__ double del64_brems(const double* el, double m, double
   } else if (v < 0.1) {
     sr = 0.1642 + 132.573 * v - 585.361 * v * v + 1407.77 * v * v * v;
   } else {
-    const double t = log(1.0 - v), lv = log(v);
+    const double t = log64(1.0 - v), lv = log64(v);
     if (v < 0.9)
       sr = -2.8922 - 19.0156 * v + 57.698 * v * v - 63.418 * v * lv + 14.1166 * t + 1.84206 * t * t;
     else
@@ -741,7 +753,7 @@ static __device__ __noinline__ double del64_sum(const double* eld, int nel, doub
     const double x0 = 1.0 - 4.0 * kElectronMass / q, x1 = 1.0 - 6.0 / (gamma * (gamma - q / mass));
     const double ri = 1.0 - sqrt(x0) * x1;
     pair = x0 > 0.0 && x1 > 0.0 && ri > 0.0 && ri < 1.0;
-    if (pair) tmin = log(ri);
+    if (pair) tmin = log64(ri);
   }
   const bool photo = pos && photo_range(1.0, 1.0, mass, K, q, &lmin, &dx);
   if (lane < 12) {
@@ -753,8 +765,8 @@ static __device__ __noinline__ double del64_sum(const double* eld, int nel, doub
   const double me_m = kMeMeV / (mass * 1e3);
   for (int e = lane; e < nel; e += 32) {
     const double* el = eld + e * kEldStride;
-    const double z1 = 0.073 * log(eom / (1.0 + el[EL_G1] * eom)) - 0.26;
-    const double z2 = 0.058 * log(eom / (1.0 + el[EL_G2] * eom)) - 0.14;
+    const double z1 = 0.073 * log64(f64::div(eom, 1.0 + el[EL_G1] * eom)) - 0.26;
+    const double z2 = 0.058 * log64(f64::div(eom, 1.0 + el[EL_G2] * eom)) - 0.14;
     const double zeta = (z1 > 0.0 && z2 > 0.0) ? z1 / z2 : 0.0;
     const bool in = el[EL_Z] > 0.0 && el[EL_A] > 0.0;
     // the pair DCS of an element vanishes at the kinematic limit
@@ -784,7 +796,7 @@ static __device__ __noinline__ double del64_sum(const double* eld, int nel, doub
     const double* o = ph + p * kPhotoPt;
     double w = 0.0;
     if (photo && el[EL_Z] > 0.0 && el[EL_A] > 0.0) {
-      const double Z = el[EL_Z], sh = Z != 1.0 && o[2] != 0.0 ? exp(o[2] * el[EL_LOGA]) : 1.0;
+      const double Z = el[EL_Z], sh = Z != 1.0 && o[2] != 0.0 ? exp64(o[2] * el[EL_LOGA]) : 1.0;
       w = fmax(o[0] * sh * (Z + (el[EL_A] - Z) * o[1]), 0.0);
     }
     item[f] = w;
@@ -1038,6 +1050,15 @@ static __device__ __noinline__ bool mixed_run(const Med<R>& m, const Consts& C, 
                                               Stream& g, R energy_limit) {
   return mixed_run_in<R>(m, C, s, x, g, energy_limit);
 }
+__device__ bool mixed_run64(const Med<double>& m, const Consts& C, State<double>& s, Cont<double>& x,
+                            Stream& g, double energy_limit);  // mc_fp64.cuh
+// The event loop after a served event.
+template <class R>
+__device__ __forceinline__ bool mixed_again(const Med<R>& m, const Consts& C, State<R>& s, Cont<R>& x, Stream& g,
+                                            R energy_limit) {
+  if constexpr (sizeof(R) == 8) return mixed_run64(m, C, s, x, g, energy_limit);
+  else return mixed_run_in<R>(m, C, s, x, g, energy_limit);
+}
 // Starts a mixed step of `distance` m at `density`; true when it suspended.
 template <class R, bool INL = false>
 __device__ bool mixed_step(const Med<R>& m, const Consts& C, State<R>& s, R density, R distance,
@@ -1058,7 +1079,8 @@ __device__ bool mixed_step(const Med<R>& m, const Consts& C, State<R>& s, R dens
   x.r1 = s.w;
   x.r2 = energy_limit > R(0) ? fmin(energy_limit, Emax) : Emax;
   x.event = 0;
-  if constexpr (INL) return mixed_run_in<R>(m, C, s, x, g, energy_limit);
+  if constexpr (sizeof(R) == 8) return mixed_run64(m, C, s, x, g, energy_limit);
+  else if constexpr (INL) return mixed_run_in<R>(m, C, s, x, g, energy_limit);
   else return mixed_run<R>(m, C, s, x, g, energy_limit);
 }
 
@@ -1068,6 +1090,14 @@ __device__ __forceinline__ R box_muller(Stream& g) {
   R r = sqrt(R(-2) * log(uni<R>(g)));
   R phi = R(2) * R(kPi) * uni<R>(g);
   return r * sin(phi);
+}
+template <>
+__device__ __forceinline__ double box_muller<double>(Stream& g) {
+  const double u = uni<double>(g);
+  const double r = u > 0.0 ? f64::sqrt(-2.0 * log64(u)) : CUDART_INF;
+  double sn, cs;
+  f64::sincospi(2.0 * uni<double>(g) - 1.0, &sn, &cs);
+  return -r * sn;  // sin(2 pi v) = -sin(pi (2 v - 1))
 }
 template <class R>
 __device__ __forceinline__ R truncated_randn(Stream& g) {
@@ -1549,6 +1579,8 @@ __device__ __forceinline__ void csda_step(const Med<R>& m, const Consts& C, Stat
   s.E = kf;
 }
 
+#include "mc_fp64.cuh"
+
 // One history in flight: the state plus its position in the dual-mode loop
 // of src/Geometry.jl:534-672, flattened so that a thread can refill itself
 // with a new history as soon as the current one ends.
@@ -1594,23 +1626,19 @@ __device__ __forceinline__ int step_done(Hist<R>& h, const Consts& C) {
 // ahead and the local density.  FP64: the reference's operations on doubles;
 // FP32: the altitude pairs and FP32 arithmetic.
 __device__ __forceinline__ bool outside(double z, double H) {
-  return z < 0.0 || z >= H - kEps64;
+  return (z < 0.0) || !f64::lt_pos(z, H - kEps64);
 }
 __device__ __forceinline__ bool outside(F2 z, F2 H) {
   return z.h + z.l < 0.f || alt_sub(z, H) >= 0.f;
 }
-__device__ __forceinline__ bool in_air_at(double z, double thick) { return z >= thick; }
+__device__ __forceinline__ bool in_air_at(double z, double thick) { return !f64::lt_pos(z, thick); }
 __device__ __forceinline__ bool in_air_at(F2 z, F2 thick) { return alt_sub(z, thick) >= 0.f; }
 __device__ __forceinline__ void boundary(double z, double thick, double H, bool in_air, double uz,
                                          double rho, double* tob, double* dens) {
   const double eps = kEps64;
-  if (!in_air) {
-    *dens = rho;
-    *tob = uz > eps ? (thick - z) / uz : uz < -eps ? (0.0 - z) / uz : 1000.0;
-  } else {
-    *dens = 1.205 * exp(-z / 12e3);
-    *tob = uz > eps ? (H - z) / uz : uz < -eps ? (thick - z) / uz : 1000.0;
-  }
+  const double next = in_air ? H : thick, prev = in_air ? thick : 0.0;
+  *dens = in_air ? 1.205 * exp64(z * (-1.0 / 12e3)) : rho;
+  *tob = uz > eps ? f64::div(next - z, uz) : uz < -eps ? f64::div(prev - z, uz) : 1000.0;
 }
 __device__ __forceinline__ void boundary(F2 z, F2 thick, F2 H, bool in_air, float uz, float rho,
                                          float* tob, float* dens) {
@@ -1627,14 +1655,9 @@ __device__ __forceinline__ void boundary_porous(double z, double thick, double H
                                                 bool in_air, bool in_p, double uz, double rho,
                                                 double prho, double* tob, double* dens) {
   const double eps = kEps64;
-  if (!in_air) {
-    *dens = in_p ? prho : rho;
-    const double next = z < pz ? pz : thick, prev = in_p ? pz : 0.0;
-    *tob = uz > eps ? (next - z) / uz : uz < -eps ? (prev - z) / uz : 1000.0;
-  } else {
-    *dens = 1.205 * exp(-z / 12e3);
-    *tob = uz > eps ? (H - z) / uz : uz < -eps ? (thick - z) / uz : 1000.0;
-  }
+  const double next = in_air ? H : (z < pz ? pz : thick), prev = in_air ? thick : (in_p ? pz : 0.0);
+  *dens = in_air ? 1.205 * exp64(z * (-1.0 / 12e3)) : (in_p ? prho : rho);
+  *tob = uz > eps ? f64::div(next - z, uz) : uz < -eps ? f64::div(prev - z, uz) : 1000.0;
 }
 __device__ __forceinline__ void boundary_porous(F2 z, F2 thick, F2 H, F2 pz, bool in_air,
                                                 bool in_p, float uz, float rho, float prho,
@@ -1694,7 +1717,10 @@ __device__ __forceinline__ int advance(const Med<R>& rock, const Med<R>& air, co
       h.need_mode = false;
     }
     const bool at_limit = sizeof(R) == 8 ? double(s.E) >= double(h.limit) - eps : s.E >= h.limit;
-    if (h.inner >= 50000 || outside(s.z, h.H) || at_limit || !(s.w > R(0)) || !isfinite(s.w)) {
+    bool dead;
+    if constexpr (sizeof(R) == 8) dead = !positive_finite(s.w);
+    else dead = !(s.w > R(0)) || !isfinite(s.w);
+    if (h.inner >= 50000 || outside(s.z, h.H) || at_limit || dead) {
       h.need_mode = true;
       continue;
     }
@@ -1711,22 +1737,39 @@ __device__ __forceinline__ int advance(const Med<R>& rock, const Med<R>& air, co
       boundary(s.z, h.thick, h.H, in_air, uz, h.rho, &tob, &rd);
     }
     const Med<R>& m = med == 0 ? rock : (POR && med == 2 ? *porous : air);
-    Loc<R> Li = locate(m, s.E);
-    R Xi = at(m, Li, MC_CR);
-    R lim = R(0.01) * Xi / fmax(rd, R(1e-6));
+    Loc<R> Li;
+    R lE = R(0), lim;  // FP64: the logarithm of the energy serves the whole step
+    if constexpr (sizeof(R) == 8) {
+      lE = log64(s.E);
+      Li = locate_log(m, s.E, lE);
+      lim = f64::div(0.01 * at(m, Li, MC_CR), f64::max_pos(rd, 1e-6));
+    } else {
+      Li = locate(m, s.E);
+      R Xi = at(m, Li, MC_CR);
+      lim = R(0.01) * Xi / fmax(rd, R(1e-6));
+    }
     // transport path at the start: the scattering step limit, then the soft
     // scattering of the step
     const R lb0 = h.scat ? transport_path(m, Li) : R(0);
     if (h.scat) {
       const R lb1 = lb0;
-      if (lb1 > R(0) && rd > R(0)) lim = fmin(lim, R(0.01) * lb1 / rd);
+      if constexpr (sizeof(R) == 8) {
+        if (lb1 > 0.0 && rd > 0.0) lim = f64::min_pos(lim, f64::div(0.01 * lb1, rd));
+      } else {
+        if (lb1 > R(0) && rd > R(0)) lim = fmin(lim, R(0.01) * lb1 / rd);
+      }
     }
     if (in_air) lim = fmin(lim, R(0.05 * 12e3) / fmax(fabs(uz), R(0.05)));
     R step = fmin(tob + R(1e-7), lim);
     step = fmin(fmax(step, R(kStepMin)), R(1000));
     if (PHASE == 0 && h.strag) {
       if constexpr (PHASE == 0) {
-        if (straggled_step<R>(m, C, s, Li, lb0, rd, step, g, h.scat, h.limit, h.x)) {
+        bool waits;
+        if constexpr (sizeof(R) == 8)
+          waits = straggled_step64<false>(m, C, s, Li, lE, lb0, rd, step, g, h.scat, h.limit, h.x);
+        else
+          waits = straggled_step<R>(m, C, s, Li, lb0, rd, step, g, h.scat, h.limit, h.x);
+        if (waits) {
           h.x.kind = CONT_STRAG;
           h.x.medium = med;
           return ADV_WAIT;
@@ -1766,7 +1809,7 @@ __device__ int resume(const Med<R>& rock, const Med<R>& air, const Med<R>* porou
       mixed_end(h.s, x, Emax, h.limit, false);
     } else {
       ++x.event;
-      if (mixed_run_in<R>(m, C, h.s, x, g, h.limit)) {
+      if (mixed_again(m, C, h.s, x, g, h.limit)) {
         x.kind = CONT_MIXED;
         return ADV_WAIT;
       }

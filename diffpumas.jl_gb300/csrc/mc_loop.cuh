@@ -269,21 +269,32 @@ __device__ __forceinline__ void serve_cta(const G& geo, const Consts& C, float* 
   }
 }
 
-// Whether this thread of the FP64 transport takes histories, for n of them on
-// a grid of `warps` warps.  An FP64 warp instruction holds its SM partition for
-// 64 cycles with one lane active as with 32 (measured), so a lane alone in its
-// warp costs as much as a full warp, but a history's divergent paths (hard
-// events, rejection loops) then wait for no other lane and no other warp.  So
-// the histories are spread over all warps of the grid, first one warp of every
-// CTA, then the next, and lanes are filled once every warp has one.
-// run_backward_mc, 100 m of rock: 10^3 histories 64.7 -> 37.9 ms, 10^4 78.5 ->
-// 67.0 ms against full warps on the fewest CTAs; a direction of 256 histories
-// 40.3 -> 13.3 ms.  At 10^5 histories all lanes are full and both are equal.
-__device__ __forceinline__ bool fp64_takes(long n, int lane) {
+// First hand-out of the FP64 transport: the place in the hand-out order of the
+// history this thread starts with (n or more: none); the counter then deals from
+// fp64_first(n) on.  An FP64 warp instruction holds its SM partition for 64
+// cycles with one lane active as with 32 (measured), so a lane alone in its warp
+// costs as much as a full warp, but a history's divergent paths (hard events,
+// rejection loops) then wait for no other lane.  So the histories are spread over
+// all warps of the grid, first one warp of every CTA, then the next, and lanes
+// are filled once every warp has one.  The places are dealt by warp and not by
+// arrival: longest first, the CTAs that arrive first would hold all the long
+// histories and the other SMs would idle at the end.  run_backward_mc, 100 m of
+// rock: 10^3 histories 64.7 -> 37.9 ms against full warps on the fewest CTAs (with
+// the steps and sums of that build); dealt by warp and not by arrival, 10^4 36.5
+// -> 29.7 ms and 5 10^4 through a mixture 85 -> 62 ms.
+__device__ __forceinline__ long fp64_per_warp(long n) {
   const long warps = long(gridDim.x) * (blockDim.x >> 5);
-  const long l = n <= warps ? 1 : (n + warps - 1) / warps;
-  const long rank = long(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  return l >= 32 || (lane < l && rank * l + lane < n);
+  return n >= 32 * warps ? 32 : (n <= warps ? 1 : (n + warps - 1) / warps);
+}
+__device__ __forceinline__ long fp64_first(long n) {
+  const long first = long(gridDim.x) * (blockDim.x >> 5) * fp64_per_warp(n);
+  return first < n ? first : n;
+}
+__device__ __forceinline__ long fp64_place(long n) {
+  const long l = fp64_per_warp(n), w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // every other row of warps runs backwards over the CTAs
+  const long rank = w * gridDim.x + ((w & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+  return lane < l ? rank * l + lane : n;
 }
 
 // Runs histories until none is left for this phase.  counter[PHASE] hands out
@@ -306,8 +317,7 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
   const long n = PHASE == 0 ? geo.n0() : long(*(volatile unsigned long long*)(counter + 2));
   typename G::Hist h;
   Stream g;
-  auto take = [&](long* idx) -> bool {
-    const long j = next_history(counter + PHASE);
+  auto begin = [&](long j, long* idx) -> bool {
     if (j >= n) return false;
     const long k = order ? long(order[j]) : j;
     if (PHASE == 0) {
@@ -317,6 +327,10 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
       *idx = geo.load(queue[k], h, g);
     }
     return true;
+  };
+  auto take = [&](long* idx) -> bool {
+    const long j = next_history(counter + PHASE);
+    return begin(sizeof(R) == 8 ? fp64_first(n) + j : j, idx);
   };
   // after a step: end the history, hand it to phase 1, or keep going
   auto settle = [&](int r, long* idx) -> bool {
@@ -409,7 +423,7 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
     // on the terms of the event's sum (del64_sum)
     const int lane = threadIdx.x & 31;
     double* buf = reinterpret_cast<double*>(coop + size_t(threadIdx.x >> 5) * stride);
-    bool live = fp64_takes(n, lane) && take(&i);
+    bool live = begin(fp64_place(n), &i);
     while (__any_sync(0xffffffffu, live)) {
       unsigned want = __ballot_sync(0xffffffffu, live && h.x.kind != CONT_NONE);
       while (want) {
