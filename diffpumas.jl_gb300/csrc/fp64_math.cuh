@@ -32,6 +32,14 @@ __device__ __forceinline__ double from_int(int k) {
   return __hiloint2double(0x43300000, int(uint32_t(k) ^ 0x80000000u)) - 4503601774854144.0;
 }
 
+// A float as a double: integer work for normal values instead of a conversion.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return double(f);  // zero, subnormal, infinity, NaN
+  return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), int(u << 29));
+}
+__device__ __forceinline__ double widen(double d) { return d; }
+
 // log x, x normal and positive: 10 FP64 instructions.  x = 2^k m with m / c in
 // [1 - 2^-9, 1 + 2^-9] of the table's c; c = 1 around x = 1, where the result
 // is the polynomial alone.

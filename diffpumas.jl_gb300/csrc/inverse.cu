@@ -19,6 +19,8 @@
 #include <cmath>
 #include <vector>
 
+#include "buckets.cuh"
+#include "fp64_math.cuh"
 #include "internal.h"
 
 namespace dp {
@@ -27,21 +29,39 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kRedBlocks = 304;  // 2 x 152 SMs for the reduction partials
 
-// y_i = sum_j J_ij x_j over the row's cells (side-exit entries excluded);
-// one warp per row.
+// y_i = sum_j J_ij x_j over the row's cells (side-exit entries excluded).
+// Eight lanes per row: the FP64 pipe bounds it, and a warp per row of some 100
+// entries spends more instructions on its tree than on its products; four entries
+// per lane are in flight at once.  6.5 10^6 entries, 65536 rows: 48 us,
+// the FP64 pipe 76% busy, against 64 us for a warp per row.
+constexpr int kRowLanes = 8;
 template <class V>
 __global__ void spmv_kernel(const int64_t* row_ptr, const int32_t* cell, const V* val,
                             const double* x, long n_rows, const double* wt, double* y) {
-  long r = (blockIdx.x * long(blockDim.x) + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (r >= n_rows) return;
+  const long r = (blockIdx.x * long(blockDim.x) + threadIdx.x) / kRowLanes;
+  const int lane = threadIdx.x % kRowLanes;
   double s = 0.0;
-  for (int64_t p = row_ptr[r] + lane, e = row_ptr[r + 1]; p < e; p += 32) {
-    int c = cell[p];
-    if (c >= 0) s += double(val[p]) * x[c];
+  if (r < n_rows) {
+    const int64_t e = row_ptr[r + 1];
+    for (int64_t p = row_ptr[r] + lane; p < e; p += 4 * kRowLanes) {
+      int c[4];
+      V v[4];
+      double xc[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t q = p + k * kRowLanes;
+        c[k] = q < e ? cell[q] : -1;
+        v[k] = q < e ? val[q] : V(0);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) xc[k] = c[k] >= 0 ? x[c[k]] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c[k] >= 0) s = fma(f64::widen(v[k]), xc[k], s);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[r] = wt ? wt[r] * s : s;
+  for (int o = kRowLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0 && r < n_rows) y[r] = wt ? wt[r] * s : s;
 }
 
 // Row sums of |J| (SART's D_row; zero rows count as 1).
@@ -63,61 +83,66 @@ __global__ void rowabs_kernel(const int64_t* row_ptr, const int32_t* cell, const
 // A ray can cross a cell in several segments: J_ij is the sum of its
 // segments' entries, which sit next to each other in the bucket (ordered by
 // entry index), so runs of one row are merged before squaring.
-// One thread per cell with at most kBigBucket entries; the larger buckets
-// (the cells next to a detector, crossed by thousands of rays) go to
-// colsum_big_kernel.
-constexpr int kBigBucket = 32;  // the bucket split of the J^T v gather (tomo.cu)
+// The entries are dealt as in the J^T v gather; the lane that meets a run's first
+// entry sums the run.  Same entries: 153 us against 118 + 84 us for a thread per
+// cell and a block per large bucket.
 template <class V>
-__global__ void colsum_kernel(const int64_t* cptr, const int32_t* perm, const V* val,
-                              const int32_t* prow, const double* wt, long ncell, int mode,
-                              double* out) {
-  long c = blockIdx.x * long(blockDim.x) + threadIdx.x;
-  if (c >= ncell) return;
-  if (cptr[c + 1] - cptr[c] > kBigBucket) return;
-  double s = 0.0, run = 0.0;
-  int row = -1;
-  for (int64_t p = cptr[c], e = cptr[c + 1]; p < e; ++p) {
-    const int r = prow[p];
-    if (r != row) {
-      if (row >= 0) s += mode == 0 ? fabs(run) : (wt ? wt[row] : 1.0) * run * run;
-      row = r;
-      run = 0.0;
-    }
-    run += double(val[perm ? perm[p] : p]);
-  }
-  if (row >= 0) s += mode == 0 ? fabs(run) : (wt ? wt[row] : 1.0) * run * run;
-  out[c] = mode == 0 ? (s > 0.0 ? s : 1.0) : s;
-}
-// A block of kBigThreads per large bucket: the bucket is cut into
-// kBigThreads contiguous chunks and each run of one row belongs to the thread
-// whose chunk it starts in (a thread skips the tail of the run entering its
-// chunk and finishes its last run past the chunk end), so every run is merged
-// before squaring, as above; the threads' sums combine in a fixed order.
-template <class V>
-__global__ void __launch_bounds__(kBigThreads) colsum_big_kernel(
-    const int64_t* cptr, const int32_t* perm, const V* val, const int32_t* prow,
-    const double* wt, const int32_t* big, int mode, double* out) {
-  __shared__ double sh[kBigThreads / 32];
-  const int c = big[blockIdx.x];
-  const int64_t b = cptr[c], e = cptr[c + 1];
-  const int64_t len = (e - b + kBigThreads - 1) / kBigThreads;
-  int64_t p = b + threadIdx.x * len;
-  const int64_t stop = p + len < e ? p + len : e;
+__global__ void __launch_bounds__(kBucketThreads) colsum_kernel(const int64_t* cptr, const V* val,
+                                                                const int32_t* prow, const double* wt, long ncell,
+                                                                int mode, const int32_t* big, int n_big,
+                                                                double* out) {
+  __shared__ V sv[kBucketWarps][kBucketStage];
+  __shared__ int32_t sr[kBucketWarps][kBucketStage];
+  __shared__ double sw[kBucketWarps][kBucketStage];
+  __shared__ Deal deal[kBucketWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool weigh = mode != 0 && wt;
+  auto add = [&](double run, double w, double& s) {
+    if (mode == 0) s += fabs(run);
+    else s = fma(w * run, run, s);
+  };
+  if (big_buckets(cptr, big, n_big, [&](int64_t b, int64_t e, int64_t first, int stride) {
+        double s = 0.0;
+        for (int64_t p = first; p < e; p += stride) {
+          const int r = prow[p];
+          const double w = weigh ? wt[r] : 1.0;
+          if (p > b && prow[p - 1] == r) continue;
+          double run = f64::widen(val[p]);
+          for (int64_t q = p + 1; q < e && prow[q] == r; ++q) run += f64::widen(val[q]);
+          add(run, w, s);
+        }
+        return s;
+      }, [&](int c, double s) { out[c] = mode == 0 ? (s > 0.0 ? s : 1.0) : s; }))
+    return;
+  const Cells C = small_cells(cptr, ncell, n_big);
   double s = 0.0;
-  if (p < stop) {
-    if (p > b) {
-      const int prev = prow[p - 1];
-      while (p < stop && prow[p] == prev) ++p;
-    }
-    while (p < stop) {
+  if (C.n <= kBucketStage) {
+    V v[8];
+    int32_t r[8];
+    stage_entries(C, deal[warp], [&](int k, int64_t p, bool ok) {
+      v[k] = ok ? val[p] : V(0);
+      r[k] = ok ? prow[p] : 0;
+    }, [&](int k, int at) {
+      sv[warp][at] = v[k];
+      sr[warp][at] = r[k];
+      sw[warp][at] = weigh ? wt[r[k]] : 1.0;
+    });
+    s = deal_entries(C, deal[warp], [&](int k, int begin, int end, double& t) {
+      const int r = sr[warp][k];
+      if (k > begin && sr[warp][k - 1] == r) return;
+      double run = f64::widen(sv[warp][k]);
+      for (int q = k + 1; q < end && sr[warp][q] == r; ++q) run += f64::widen(sv[warp][q]);
+      add(run, sw[warp][k], t);
+    });
+  } else {
+    for (int64_t p = C.b; p < C.e;) {
       const int r = prow[p];
       double run = 0.0;
-      for (; p < e && prow[p] == r; ++p) run += double(val[perm ? perm[p] : p]);
-      s += mode == 0 ? fabs(run) : (wt ? wt[r] : 1.0) * run * run;
+      for (; p < C.e && prow[p] == r; ++p) run += f64::widen(val[p]);
+      add(run, weigh ? wt[r] : 1.0, s);
     }
   }
-  s = big_block_sum(s, sh);
-  if (threadIdx.x == 0) out[c] = mode == 0 ? (s > 0.0 ? s : 1.0) : s;
+  if (C.cell >= 0 && !C.big) out[C.cell] = mode == 0 ? (s > 0.0 ? s : 1.0) : s;
 }
 
 // Fixed-order dot product: block partials, then one block.
@@ -177,12 +202,12 @@ __global__ void sart_update_kernel(double* rho, const double* g, const double* c
 
 // Conjugate-gradient pieces with device-resident scalars (no host round trip
 // inside the CG loop).  s[0] = r.z, s[1] = p.Ap, s[2] = new r.z.
-__global__ void cg_init_kernel(const double* g, const double* prec, long n, double* x, double* r,
+__global__ void cg_init_kernel(const double* g, const double* iprec, long n, double* x, double* r,
                                double* z, double* p) {
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n;
        i += long(gridDim.x) * blockDim.x) {
     double ri = -g[i];
-    double zi = ri / prec[i];
+    double zi = ri * iprec[i];
     x[i] = 0.0;
     r[i] = ri;
     z[i] = zi;
@@ -196,14 +221,16 @@ __global__ void trial_kernel(const double* rho, const double* d, long n, double 
        i += long(gridDim.x) * blockDim.x)
     out[i] = fmin(fmax(rho[i] + alpha * d[i], lo), hi);
 }
-// prec = max(diag, floor) (Jacobi preconditioner) and damp = mu max(diag, floor)
-__global__ void lm_diag_kernel(const double* diag, long n, double floor_, double mu, double* prec,
+// iprec = 1 / ((1 + mu) max(diag, floor)) (Jacobi preconditioner, inverted once
+// per system: a division takes nine FP64 instructions and every CG step applies
+// it) and damp = mu max(diag, floor)
+__global__ void lm_diag_kernel(const double* diag, long n, double floor_, double mu, double* iprec,
                                double* damp) {
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n;
        i += long(gridDim.x) * blockDim.x) {
     double d = fmax(diag[i], floor_);
     damp[i] = mu * d;
-    prec[i] = (1.0 + mu) * d;
+    iprec[i] = 1.0 / ((1.0 + mu) * d);
   }
 }
 __global__ void max_part_kernel(const double* a, long n, double* part) {
@@ -241,8 +268,19 @@ __device__ __forceinline__ int degree(Dims d, long c, int* nb) {
 // -y, +y, -z, +z (no neighbour array, so nothing goes to local memory)
 __device__ __forceinline__ double lap_sum(const double* x, Dims d, long c) {
   const long sxy = long(d.nx) * d.ny;
-  const long k = c / sxy, rem = c - k * sxy;
-  const int j = int(rem / d.nx), i = int(rem - long(j) * d.nx);
+  int i, j, k;
+  if (d.nz * sxy <= 0xffffffffll) {  // 32-bit divisions
+    const uint32_t q = uint32_t(c), s = uint32_t(sxy);
+    k = int(q / s);
+    const uint32_t rem = q - uint32_t(k) * s;
+    j = int(rem / uint32_t(d.nx));
+    i = int(rem - uint32_t(j) * uint32_t(d.nx));
+  } else {
+    k = int(c / sxy);
+    const long rem = c - k * sxy;
+    j = int(rem / d.nx);
+    i = int(rem - long(j) * d.nx);
+  }
   const double xc = x[c];
   double s = 0.0;
   if (i > 0) s += xc - x[c - 1];
@@ -286,23 +324,36 @@ __global__ void __launch_bounds__(kThreads) cg_apply_kernel(const double* p, con
   }
   block_part(s, sh, part);
 }
-// x += a p, r -= a Ap, z = r / prec with a = s[0] / s[1], and the block
+// x += a p, r -= a Ap, z = r iprec with a = s[0] / s[1], and the block
 // partials of r . z (same traversal as above).
 __global__ void __launch_bounds__(kThreads) cg_step_dot_kernel(const double* s, const double* p,
                                                                const double* Ap,
-                                                               const double* prec, long n,
+                                                               const double* iprec, long n,
                                                                double* x, double* r, double* z,
                                                                double* part) {
   __shared__ double sh[kThreads];
   const double a = s[1] != 0.0 ? s[0] / s[1] : 0.0;
   double acc = 0.0;
-  for (long i = blockIdx.x * long(kThreads) + threadIdx.x; i < n; i += long(gridDim.x) * kThreads) {
-    x[i] += a * p[i];
-    const double ri = r[i] - a * Ap[i];
-    r[i] = ri;
-    const double zi = ri / prec[i];
-    z[i] = zi;
+  auto one = [&](double& xi, double pi, double& ri, double Api, double qi, double& zi) {
+    xi += a * pi;
+    ri -= a * Api;
+    zi = ri * qi;
     acc += ri * zi;
+  };
+  // two cells at a time (the vectors are 256-byte aligned): bound by memory
+  for (long i = 2 * (blockIdx.x * long(kThreads) + threadIdx.x); i < n; i += 2 * long(gridDim.x) * kThreads) {
+    if (i + 1 < n) {
+      const double2 pv = *reinterpret_cast<const double2*>(p + i), Av = *reinterpret_cast<const double2*>(Ap + i);
+      const double2 qv = *reinterpret_cast<const double2*>(iprec + i);
+      double2 xv = *reinterpret_cast<double2*>(x + i), rv = *reinterpret_cast<double2*>(r + i), zv;
+      one(xv.x, pv.x, rv.x, Av.x, qv.x, zv.x);
+      one(xv.y, pv.y, rv.y, Av.y, qv.y, zv.y);
+      *reinterpret_cast<double2*>(x + i) = xv;
+      *reinterpret_cast<double2*>(r + i) = rv;
+      *reinterpret_cast<double2*>(z + i) = zv;
+    } else {
+      one(x[i], p[i], r[i], Ap[i], iprec[i], z[i]);
+    }
   }
   block_part(acc, sh, part);
 }
@@ -501,7 +552,7 @@ struct Solver {
     return h;
   }
   int spmv(const double* x, const double* wt, double* y) {
-    int blocks = int((n_rays * 32 + kThreads - 1) / kThreads);
+    int blocks = int((n_rays * kRowLanes + kThreads - 1) / kThreads);
     timed_begin(ctx);
     if (precision)
       spmv_kernel<float><<<blocks, kThreads, 0, ctx->stream>>>(pa->row_ptr, pa->cell,
@@ -519,24 +570,14 @@ struct Solver {
     return tomo_transpose(ctx, pa, jcsc, precision, u, out, true);
   }
   int colsum(const double* wt, int mode, double* out) {
-    int blocks = int((ncell + kThreads - 1) / kThreads);
+    const int blocks = bucket_blocks(ncell, pa->n_big);
     timed_begin(ctx);
-    if (precision) {
-      const float* v = static_cast<const float*>(jcsc);
-      colsum_kernel<float><<<blocks, kThreads, 0, ctx->stream>>>(pa->cptr, nullptr, v, pa->prow,
-                                                                 wt, ncell, mode, out);
-      if (pa->n_big > 0)
-        colsum_big_kernel<float><<<pa->n_big, kBigThreads, 0, ctx->stream>>>(
-            pa->cptr, nullptr, v, pa->prow, wt, pa->big, mode, out);
-    } else {
-      const double* v = static_cast<const double*>(jcsc);
-      colsum_kernel<double><<<blocks, kThreads, 0, ctx->stream>>>(pa->cptr, nullptr, v, pa->prow,
-                                                                  wt, ncell, mode, out);
-      if (pa->n_big > 0)
-        colsum_big_kernel<double><<<pa->n_big, kBigThreads, 0, ctx->stream>>>(
-            pa->cptr, nullptr, v, pa->prow, wt, pa->big, mode, out);
-    }
-    if (pa->n_big > 0) ++ctx->launches;
+    if (precision)
+      colsum_kernel<float><<<blocks, kBucketThreads, 0, ctx->stream>>>(
+          pa->cptr, static_cast<const float*>(jcsc), pa->prow, wt, ncell, mode, pa->big, pa->n_big, out);
+    else
+      colsum_kernel<double><<<blocks, kBucketThreads, 0, ctx->stream>>>(
+          pa->cptr, static_cast<const double*>(jcsc), pa->prow, wt, ncell, mode, pa->big, pa->n_big, out);
     DP_CHECK_CUDA(ctx, cudaGetLastError());
     timed_end(ctx, "gn_colsum");
     return DP_OK;

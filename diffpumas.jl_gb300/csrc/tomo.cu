@@ -35,6 +35,7 @@
 #include <string>
 #include <vector>
 
+#include "buckets.cuh"
 #include "fp64_math.cuh"
 #include "internal.h"
 
@@ -240,7 +241,6 @@ __global__ void place_kernel(const int32_t* col, long nnz, const int64_t* cptr, 
 // Buckets are ordered by entry index.  Small buckets (<= kSmallBucket): one
 // thread, insertion sort.  Large ones (cells next to a detector collect one
 // entry per ray of that detector) are listed and sorted by a block each.
-constexpr int kSmallBucket = 32;
 __global__ void sort_small_buckets_kernel(const int64_t* cptr, long ncell, int32_t* perm,
                                           int32_t* big, int32_t* n_big) {
   long c = blockIdx.x * long(blockDim.x) + threadIdx.x;
@@ -579,34 +579,61 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
   }
 }
 
-// J^T r over the precomputed CSC permutation of a large bucket: one block of
-// kBigThreads per cell; thread t sums entries t, t + kBigThreads, ... in
-// order, then big_block_sum -- the same arithmetic order on every call.
+// J^T r over the precomputed CSC permutation, every bucket in a fixed order
+// (buckets.cuh).  A warp loads the entries of its 32 cells together, so that the
+// dependent gathers of the rows' cotangents are all in flight; FP32 values are
+// widened by integer work (a conversion holds the FP64 pipe like the
+// multiply-add).  6.5 10^6 entries in 10^6 cells, 13378 of them large:
+// 71 us against 66 + 32 us for a thread per cell and then a block per large bucket.
+// What is left is the latency of the gathers: the FP64 pipe is 45% busy.
 // perm == nullptr: the values are already in CSC order.
 template <class V>
-__global__ void __launch_bounds__(kBigThreads) gather_big_kernel(
-    const int64_t* cptr, const int32_t* perm, const V* val, const int32_t* prow,
-    const double* cot, const int32_t* big, int n_big, double* grad) {
-  __shared__ double sh[kBigThreads / 32];
-  const int c = big[blockIdx.x];
+__global__ void __launch_bounds__(kBucketThreads) gather_kernel(const int64_t* cptr, const int32_t* perm,
+                                                                const V* val, const int32_t* prow,
+                                                                const double* cot, long ncell,
+                                                                const int32_t* big, int n_big, double* grad) {
+  __shared__ V sv[kBucketWarps][kBucketStage];
+  __shared__ double sc[kBucketWarps][kBucketStage];
+  __shared__ Deal deal[kBucketWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (big_buckets(cptr, big, n_big, [&](int64_t b, int64_t e, int64_t first, int stride) {
+        double s = 0.0;
+        const int64_t mine = first - b;
+        for (int64_t p = b; p < e; p += 4 * stride) {
+          V v[4];
+          double c[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int64_t q = p + k * stride + mine;
+            v[k] = q < e ? val[perm ? perm[q] : q] : V(0);
+            c[k] = q < e ? cot[prow[q]] : 0.0;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (p + k * stride < e) s = fma(f64::widen(v[k]), c[k], s);
+        }
+        return s;
+      }, [&](int c, double s) { grad[c] = s; }))
+    return;
+  const Cells C = small_cells(cptr, ncell, n_big);
   double s = 0.0;
-  for (int64_t p = cptr[c] + threadIdx.x, e = cptr[c + 1]; p < e; p += kBigThreads)
-    s += double(val[perm ? perm[p] : p]) * cot[prow[p]];
-  s = big_block_sum(s, sh);
-  if (threadIdx.x == 0) grad[c] = s;
-}
-// Cells with at most kSmallBucket entries: one thread, entries in order.
-template <class V>
-__global__ void gather_small_kernel(const int64_t* cptr, const int32_t* perm, const V* val,
-                                    const int32_t* prow, const double* cot, long ncell,
-                                    double* grad) {
-  long c = blockIdx.x * long(blockDim.x) + threadIdx.x;
-  if (c >= ncell) return;
-  int64_t b = cptr[c], e = cptr[c + 1];
-  if (e - b > kSmallBucket) return;  // gather_big_kernel
-  double s = 0.0;
-  for (int64_t p = b; p < e; ++p) s += double(val[perm ? perm[p] : p]) * cot[prow[p]];
-  grad[c] = s;
+  if (C.n <= kBucketStage) {
+    V v[8];
+    int32_t r[8];
+    stage_entries(C, deal[warp], [&](int k, int64_t p, bool ok) {
+      v[k] = ok ? val[perm ? perm[p] : p] : V(0);
+      r[k] = ok ? prow[p] : 0;
+    }, [&](int k, int at) {
+      sv[warp][at] = v[k];
+      sc[warp][at] = cot[r[k]];
+    });
+    s = deal_entries(C, deal[warp], [&](int k, int, int, double& t) {
+      t = fma(f64::widen(sv[warp][k]), sc[warp][k], t);
+    });
+  } else {
+    for (int64_t p = C.b; p < C.e; ++p) s = fma(f64::widen(val[perm ? perm[p] : p]), cot[prow[p]], s);
+  }
+  if (C.cell >= 0 && !C.big) grad[C.cell] = s;
 }
 // The Jacobian values of the bucketed entries in CSC order (out[p] =
 // val[perm[p]] for p < *n_bucketed), so that repeated J^T v products read
@@ -1007,22 +1034,13 @@ int tomo_transpose(dp_ctx* ctx, const dp_paths* pa, const void* jbuf, int precis
   const int32_t* perm = csc ? nullptr : pa->perm;
   {
     timed_begin(ctx);
-    if (precision == 0) {
-      const double* v = static_cast<const double*>(jbuf);
-      gather_small_kernel<double><<<int((ncell + 255) / 256), 256, 0, ctx->stream>>>(
-          pa->cptr, perm, v, pa->prow, cot, ncell, grad);
-      if (pa->n_big > 0)
-        gather_big_kernel<double><<<pa->n_big, kBigThreads, 0, ctx->stream>>>(
-            pa->cptr, perm, v, pa->prow, cot, pa->big, pa->n_big, grad);
-    } else {
-      const float* v = static_cast<const float*>(jbuf);
-      gather_small_kernel<float><<<int((ncell + 255) / 256), 256, 0, ctx->stream>>>(
-          pa->cptr, perm, v, pa->prow, cot, ncell, grad);
-      if (pa->n_big > 0)
-        gather_big_kernel<float><<<pa->n_big, kBigThreads, 0, ctx->stream>>>(
-            pa->cptr, perm, v, pa->prow, cot, pa->big, pa->n_big, grad);
-    }
-    ctx->launches += pa->n_big > 0 ? 1 : 0;
+    const int blocks = bucket_blocks(ncell, pa->n_big);
+    if (precision == 0)
+      gather_kernel<double><<<blocks, kBucketThreads, 0, ctx->stream>>>(
+          pa->cptr, perm, static_cast<const double*>(jbuf), pa->prow, cot, ncell, pa->big, pa->n_big, grad);
+    else
+      gather_kernel<float><<<blocks, kBucketThreads, 0, ctx->stream>>>(
+          pa->cptr, perm, static_cast<const float*>(jbuf), pa->prow, cot, ncell, pa->big, pa->n_big, grad);
     DP_CHECK_CUDA(ctx, cudaGetLastError());
     timed_end(ctx, "tomo_transpose");
   }
@@ -1426,14 +1444,9 @@ extern "C" int dp_tomo_eval_noalloc_dev(dp_ctx* ctx, const dp_physics* ph, const
   DP_CHECK_CUDA(ctx, cudaGetLastError());
   if (adj) {
     const long ncell = long(pa->grid.nx) * pa->grid.ny * pa->grid.nz;
-    gather_small_kernel<float><<<int((ncell + 255) / 256), 256, 0, ctx->stream>>>(
-        pa->cptr, pa->perm, jac, pa->prow, cot, ncell, grad);
+    gather_kernel<float><<<bucket_blocks(ncell, pa->n_big), kBucketThreads, 0, ctx->stream>>>(
+        pa->cptr, pa->perm, jac, pa->prow, cot, ncell, pa->big, pa->n_big, grad);
     ++ctx->launches;
-    if (pa->n_big > 0) {
-      gather_big_kernel<float><<<pa->n_big, kBigThreads, 0, ctx->stream>>>(
-          pa->cptr, pa->perm, jac, pa->prow, cot, pa->big, pa->n_big, grad);
-      ++ctx->launches;
-    }
     DP_CHECK_CUDA(ctx, cudaGetLastError());
   }
   return check(ctx);
