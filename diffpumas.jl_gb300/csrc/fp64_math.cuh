@@ -74,6 +74,15 @@ __device__ __forceinline__ double rcp(double x) {
   return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ double div(double a, double b) { return a * rcp(b); }
+// a / b correctly rounded, y = __drcp_rn(b): 5 FP64 instructions.  Markstein,
+// "IA-64 and Elementary Functions" (2000): a quotient within one unit, corrected
+// by its exact remainder times the rounded reciprocal, is the rounded one.  For b
+// and the quotient well inside the normal range (a tiny a keeps a tiny quotient).
+__device__ __forceinline__ double div_rn(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
+}
 
 // 1 / sqrt(x) and sqrt(x) for normal positive x: 5 and 6 FP64 instructions.
 __device__ __forceinline__ double rsqrt(double x) {
