@@ -10,6 +10,7 @@ using wt::Lane;
 using wt::Params;
 using wt::kMaxChunks;
 using wt::kThreads;
+constexpr unsigned kAll = 0xffffffffu;
 
 // ------------------------------------------------------------ N tangents
 template <int N>
@@ -194,9 +195,10 @@ __device__ __forceinline__ T<N> decay(const Consts& k, T<N> L, T<N> Eavg) {
   return texp(-L / (b * g * cst<N>(k.ctau)));
 }
 
-// One Heun step (src/Tomography.jl:455-471); false on an invalid step.
+// One Heun step (src/Tomography.jl:455-471); dedx0 becomes the stopping power at
+// its end.  False on an invalid step.
 template <int N, class SF>
-__device__ __forceinline__ bool heun(const Consts& k, SF S, T<N> dedx0, T<N> ds, T<N> density,
+__device__ __forceinline__ bool heun(const Consts& k, SF S, T<N>& dedx0, T<N> ds, T<N> density,
                                      T<N>& E, T<N>& W) {
   T<N> gx = ds * density;
   T<N> Ep = E + dedx0 * gx;
@@ -207,43 +209,58 @@ __device__ __forceinline__ bool heun(const Consts& k, SF S, T<N> dedx0, T<N> ds,
   W = W * (dedxn / tmax(dedx0, cst<N>(Real(1e-30))));
   W = W * decay(k, ds, Real(0.5) * (E + En));
   E = En;
+  dedx0 = dedxn;
   return true;
 }
 
-// propagate_csda_cell_segment / propagate_csda_uniform_segment (:444-509)
+// propagate_csda_cell_segment / propagate_csda_uniform_segment (:444-509).
+// The whole warp calls it and the lanes with `on` walk; true where the walk is
+// valid.  A direction is a chain of some 10^3 steps of 300 instructions in one warp,
+// bound by their latency: so the lanes stay together in every step (left to
+// themselves they part at the first that returns), and a step's last stopping power
+// is the next one's first.  1024 directions of 32 samples with the Jacobian: 2.38
+// ms, 3.77 ms with lanes that return alone and three stopping powers per step.
 template <int N, class SF>
-__device__ bool solid_segment(const Consts& k, SF S, T<N> density, Real distance, T<N>& E,
-                              T<N>& W) {
-  T<N> remaining = cst<N>(distance);
-  for (int guard = 0; remaining.v > Real(1e-8); ++guard) {
-    if (guard > 10000000) return false;
-    T<N> dedx0 = S(E);
-    if (!isfinite(dedx0.v) || dedx0.v <= Real(0)) return false;
-    T<N> grel = Real(wt::kMaxGain) * tmax(E, cst<N>(Real(1e-6))) / dedx0;
-    T<N> gstep = tmin(tmin(remaining * density, tmax(grel, cst<N>(Real(1e-6)))),
-                      Real(wt::kMaxStep) * density);
-    T<N> ds = tmin(remaining, gstep / tmax(density, cst<N>(Real(1e-12))));
-    if (ds.v <= Real(0)) return false;
-    if (!heun(k, S, dedx0, ds, density, E, W)) return false;
-    remaining = remaining - ds;
+__device__ __forceinline__ bool solid_segment(const Consts& k, SF S, T<N> density, Real distance, T<N>& E,
+                                              T<N>& W, bool on) {
+  T<N> remaining = cst<N>(distance), dedx0 = cst<N>(Real(0));
+  if (!(remaining.v > Real(1e-8))) return on;  // the same for the whole warp
+  dedx0 = S(E);
+  for (int guard = 0;; ++guard) {
+    const bool go = on && remaining.v > Real(1e-8);
+    if (!__any_sync(kAll, go)) return on;
+    if (go) {
+      on = false;
+      if (guard <= 10000000 && isfinite(dedx0.v) && dedx0.v > Real(0)) {
+        T<N> grel = Real(wt::kMaxGain) * tmax(E, cst<N>(Real(1e-6))) / dedx0;
+        T<N> gstep = tmin(tmin(remaining * density, tmax(grel, cst<N>(Real(1e-6)))),
+                          Real(wt::kMaxStep) * density);
+        T<N> ds = tmin(remaining, gstep / tmax(density, cst<N>(Real(1e-12))));
+        if (ds.v > Real(0)) {
+          on = heun(k, S, dedx0, ds, density, E, W);
+          remaining = remaining - ds;
+        }
+      }
+    }
   }
-  return true;
 }
 
 // propagate_csda_air_segment (:516-551): remaining and traversed carry the
 // steps' tangents, and with them the altitude of the density.
 template <int N>
 __device__ bool air_segment(const Consts& k, const Tables& tb, Real start_z, Real cos_t,
-                            Real distance, T<N>& E, T<N>& W) {
+                            Real distance, T<N>& E, T<N>& W, bool on) {
+  if (!on) return false;
   auto S = [&](T<N> e) { return at(tb, locate(tb, e), wt::A_CS); };
   T<N> remaining = cst<N>(distance), traversed = cst<N>(Real(0));
   const T<N> base = cst<N>(k.det_elev + start_z), ct = cst<N>(cos_t);
   const T<N> H = cst<N>(Real(12e3));
+  if (!(remaining.v > Real(1e-8))) return true;
+  T<N> dedx0 = S(E);
   for (int guard = 0; remaining.v > Real(1e-8); ++guard) {
     if (guard > 10000000) return false;
     T<N> alt = base + ct * (traversed + Real(0.5) * tmin(remaining, cst<N>(Real(wt::kMaxStep))));
     T<N> rho = Real(1.205) * texp(-alt / H);
-    T<N> dedx0 = S(E);
     if (!isfinite(dedx0.v) || dedx0.v <= Real(0)) return false;
     T<N> grel = Real(wt::kMaxGain) * tmax(E, cst<N>(Real(1e-6))) / dedx0;
     T<N> ds = tmin(tmin(remaining, cst<N>(Real(wt::kMaxStep))),
@@ -279,10 +296,11 @@ __device__ __forceinline__ void vh_rock(const Tables& tb, T<N> e_rep, T<N> gx, T
   h = (at(tb, a, wt::R_CS) - at(tb, a, wt::R_MS)) * gx;
 }
 
-// Pass 1: flux of one sample and its end-of-path adjoint constants.  The
-// per-segment partials are accumulated in FP64.
-__device__ Lane pass1(const Params& P, const Consts& k, const Tables& tb, long b, double E0,
-                      double q) {
+// Pass 1: flux of one sample and its end-of-path adjoint constants, the warp's
+// lanes together (those with `on` hold a sample).  The per-segment partials are
+// accumulated in FP64.
+__device__ __forceinline__ Lane pass1(const Params& P, const Consts& k, const Tables& tb, long b, double E0,
+                                      double q, bool on) {
   Lane out{0.0, 0.0, 0.0, 0.0};
   const double ct = P.cos_t[b];
   Real E = Real(E0), W = Real(1), V = Real(0), H = Real(0);
@@ -295,38 +313,43 @@ __device__ Lane pass1(const Params& P, const Consts& k, const Tables& tb, long b
     T<1> e = seed<1>(E, 0), g = cst<1>(Real(1));
     const T<1> e_in = e;
     const Real len = Real(P.seg_len[j]);
-    if (!solid_segment(k, [&](T<1> x) { return cell_S(tb, c, x); }, rho, len, e, g)) return out;
-    T<1> v, h;
-    vh_cell(tb, c, Real(0.5) * (e_in + e), len * rho, v, h);
-    Cs += double(g.d[0] / g.v) * Pk;
-    Cv += double(v.d[0]) * Pk;
-    Ch += double(h.d[0]) * Pk;
-    Pk *= double(e.d[0]);
-    E = e.v;
-    W *= g.v;
-    V += v.v;
-    H += h.v;
+    on = solid_segment(k, [&](T<1> x) { return cell_S(tb, c, x); }, rho, len, e, g, on);
+    if (on) {
+      T<1> v, h;
+      vh_cell(tb, c, Real(0.5) * (e_in + e), len * rho, v, h);
+      Cs += double(g.d[0] / g.v) * Pk;
+      Cv += double(v.d[0]) * Pk;
+      Ch += double(h.d[0]) * Pk;
+      Pk *= double(e.d[0]);
+      E = e.v;
+      W *= g.v;
+      V += v.v;
+      H += h.v;
+    }
   }
   if (P.rem[b] > 1e-8) {
     T<1> e = seed<1>(E, 0), g = cst<1>(Real(1));
     const T<1> e_in = e;
     auto S = [&](T<1> x) { return at(tb, locate(tb, x), wt::R_CS); };
-    if (!solid_segment(k, S, cst<1>(k.rho_rock), Real(P.rem[b]), e, g)) return out;
-    T<1> v, h;
-    vh_rock(tb, Real(0.5) * (e_in + e), cst<1>(Real(P.rem[b]) * k.rho_rock), v, h);
-    Cs += double(g.d[0] / g.v) * Pk;
-    Cv += double(v.d[0]) * Pk;
-    Ch += double(h.d[0]) * Pk;
-    Pk *= double(e.d[0]);
-    E = e.v;
-    W *= g.v;
-    V += v.v;
-    H += h.v;
+    on = solid_segment(k, S, cst<1>(k.rho_rock), Real(P.rem[b]), e, g, on);
+    if (on) {
+      T<1> v, h;
+      vh_rock(tb, Real(0.5) * (e_in + e), cst<1>(Real(P.rem[b]) * k.rho_rock), v, h);
+      Cs += double(g.d[0] / g.v) * Pk;
+      Cv += double(v.d[0]) * Pk;
+      Ch += double(h.d[0]) * Pk;
+      Pk *= double(e.d[0]);
+      E = e.v;
+      W *= g.v;
+      V += v.v;
+      H += h.v;
+    }
   }
   {
     T<1> e = seed<1>(E, 0), g = cst<1>(Real(1));
     const double air = fmax(0.0, P.primary - P.exit_z[b]) / fmax(ct, 1e-3);
-    if (!air_segment(k, tb, Real(P.exit_z[b]), Real(ct), Real(air), e, g)) return out;
+    on = air_segment(k, tb, Real(P.exit_z[b]), Real(ct), Real(air), e, g, on);
+    if (!on) return out;
     Cs += double(g.d[0] / g.v) * Pk;
     Pk *= double(e.d[0]);
     E = e.v;
@@ -418,9 +441,10 @@ __global__ void __launch_bounds__(kThreads) wtomo_kernel(const __grid_constant__
     for (int ch = 0; ch < kMaxChunks; ++ch) {
       L[ch] = Lane{0.0, 0.0, 0.0, 0.0};
       const int s = ch * 32 + lane;
-      if (ch < n_chunks && s < P.n_e) {
-        L[ch] = pass1(P, k, tb, b, P.E[s], P.q[s]);
-        L[ch].f *= 2.0 * P.ew[s];
+      if (ch < n_chunks) {
+        const bool on = s < P.n_e;
+        L[ch] = pass1(P, k, tb, b, on ? P.E[s] : 1.0, on ? P.q[s] : 0.0, on);
+        if (on) L[ch].f *= 2.0 * P.ew[s];
       }
       sum += L[ch].f;
     }
@@ -459,27 +483,25 @@ __global__ void __launch_bounds__(kThreads) wtomo_kernel(const __grid_constant__
       bool alive = active;
       for (int64_t j = s0; j < s1; ++j) {
         double gk = 0.0;
+        const int cell = P.seg_cell[j];
+        Cell<2> c{seed<2>(Real(P.wf[cell]), 1), wt::cell_porous(P, cell)};
+        T<2> rho = cell_density(k, c);
+        T<2> e = seed<2>(E, 0), g = cst<2>(Real(1));
+        const T<2> e_in = e;
+        const Real len = Real(P.seg_len[j]);
+        // (every walk is valid: pass 1 saw the same)
+        alive = solid_segment(k, [&](T<2> x) { return cell_S(tb, c, x); }, rho, len, e, g, alive);
         if (alive) {
-          const int cell = P.seg_cell[j];
-          Cell<2> c{seed<2>(Real(P.wf[cell]), 1), wt::cell_porous(P, cell)};
-          T<2> rho = cell_density(k, c);
-          T<2> e = seed<2>(E, 0), g = cst<2>(Real(1));
-          const T<2> e_in = e;
-          const Real len = Real(P.seg_len[j]);
-          if (solid_segment(k, [&](T<2> x) { return cell_S(tb, c, x); }, rho, len, e, g)) {
-            T<2> v, h;
-            vh_cell(tb, c, Real(0.5) * (e_in + e), len * rho, v, h);
-            Cs += double(g.d[0] / g.v) * Pk;
-            Cv += double(v.d[0]) * Pk;
-            Ch += double(h.d[0]) * Pk;
-            Pk *= double(e.d[0]);
-            const double lam = (l.A - Cs - l.aV * Cv - l.aH * Ch) / Pk;
-            gk = l.f * (lam * double(e.d[1]) + double(g.d[1] / g.v) + l.aV * double(v.d[1]) +
-                        l.aH * double(h.d[1]));
-            E = e.v;
-          } else {
-            alive = false;  // not reached: pass 1 saw the same valid walk
-          }
+          T<2> v, h;
+          vh_cell(tb, c, Real(0.5) * (e_in + e), len * rho, v, h);
+          Cs += double(g.d[0] / g.v) * Pk;
+          Cv += double(v.d[0]) * Pk;
+          Ch += double(h.d[0]) * Pk;
+          Pk *= double(e.d[0]);
+          const double lam = (l.A - Cs - l.aV * Cv - l.aH * Ch) / Pk;
+          gk = l.f * (lam * double(e.d[1]) + double(g.d[1] / g.v) + l.aV * double(v.d[1]) +
+                      l.aH * double(h.d[1]));
+          E = e.v;
         }
         gk = wt::warp_sum(gk);
         if (lane == 0) P.jac[j] = (ch ? P.jac[j] : 0.0) + scale * gk;
