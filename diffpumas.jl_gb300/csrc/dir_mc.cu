@@ -497,7 +497,7 @@ int dir_device(dp_ctx* ctx, dp_dir_media* M, int precision, dp_dir_media::Dev** 
 }
 
 template <class R, int PHASE, int T>
-int dir_phase(dp_ctx* ctx, const DirParams& P, size_t smem, long max_blocks) {
+int dir_phase(dp_ctx* ctx, const DirParams& P, size_t smem) {
   const int threads = T;
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(dir_kernel<R, PHASE, T>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -509,7 +509,7 @@ int dir_phase(dp_ctx* ctx, const DirParams& P, size_t smem, long max_blocks) {
                                                                    threads, smem));
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
   if (per_sm < 1) return fail(ctx, DP_ERR_CUDA, "fixed-path MC kernel does not fit on a multiprocessor");
-  long blocks = std::max(1L, std::min(long(per_sm) * n_sm, max_blocks));
+  long blocks = std::max(1L, std::min(long(per_sm) * n_sm, P.n));
   timed_begin(ctx);
   dir_kernel<R, PHASE, T><<<int(blocks), threads, smem, ctx->stream>>>(P);
   DP_CHECK_CUDA(ctx, cudaGetLastError());
@@ -548,15 +548,14 @@ int dir_launch_t(dp_ctx* ctx, DirParams& P) {
   }
   const size_t smem = dir_coop_offset<R>(P) + coop_bytes;
   if (smem > size_t(dev_smem)) return fail(ctx, DP_ERR_ARG, "too many media for the fixed-path MC kernel");
-  const long need = sizeof(R) == 4 ? (P.n + threads - 1) / threads : P.n;
   const long rec_blocks = std::min((P.n + 255) / 256, 152L * 32);
   DP_CHECK_CUDA(ctx, cudaMemsetAsync(P.counter, 0, 3 * sizeof(unsigned long long), ctx->stream));
   timed_begin(ctx);
   dir_init_kernel<R><<<int(rec_blocks), 256, 0, ctx->stream>>>(P);
   DP_CHECK_CUDA(ctx, cudaGetLastError());
   timed_end(ctx, "dir_init");
-  int rc = dir_phase<R, 0, T>(ctx, P, smem, need);
-  if (!rc) rc = dir_phase<R, 1, T>(ctx, P, smem, need);
+  int rc = dir_phase<R, 0, T>(ctx, P, smem);
+  if (!rc) rc = dir_phase<R, 1, T>(ctx, P, smem);
   if (rc) return rc;
   timed_begin(ctx);
   dir_finish_kernel<R><<<int(rec_blocks), 256, 0, ctx->stream>>>(P);

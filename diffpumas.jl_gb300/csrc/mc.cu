@@ -1021,7 +1021,7 @@ int group_tally(dp_ctx* ctx, const double* contrib, const int32_t* status, const
 namespace {
 
 template <class R, int PHASE, int T, bool POR>
-int launch_phase(dp_ctx* ctx, McParams& P, size_t smem, long max_blocks) {
+int launch_phase(dp_ctx* ctx, McParams& P, size_t smem) {
   const int threads = T;
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(mc_kernel<R, PHASE, T, POR>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -1033,7 +1033,7 @@ int launch_phase(dp_ctx* ctx, McParams& P, size_t smem, long max_blocks) {
                          &per_sm, mc_kernel<R, PHASE, T, POR>, threads, smem));
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
   if (per_sm < 1) return fail(ctx, DP_ERR_CUDA, "MC kernel does not fit on a multiprocessor");
-  long blocks = std::min(long(per_sm) * n_sm, max_blocks);
+  long blocks = std::min(long(per_sm) * n_sm, P.n);
   if (blocks < 1) blocks = 1;
   timed_begin(ctx);
   mc_kernel<R, PHASE, T, POR><<<int(blocks), threads, smem, ctx->stream>>>(P);
@@ -1081,7 +1081,6 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
   // the DCS buffer fills the smallest carve-out step that holds it, the rest
   // of the SM's 256 KB is L1 for the spilled stack
   smem = fit(std::min(size_t(dev_smem), carveout_cap(smem)));
-  long need = sizeof(R) == 4 ? (P.n + threads - 1) / threads : P.n;
   long rec_blocks = std::min((P.n + 255) / 256, 152L * 32);
   DP_CHECK_CUDA(ctx, cudaMemsetAsync(P.counter, 0, 3 * sizeof(unsigned long long), ctx->stream));
   timed_begin(ctx);
@@ -1095,7 +1094,7 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
     --ctx->launches;  // timed_begin counted one of the three
     timed_end(ctx, "mc_order");
   }
-  int rc = launch_phase<R, 0, T, POR>(ctx, P, smem, need);
+  int rc = launch_phase<R, 0, T, POR>(ctx, P, smem);
   if (rc) return rc;
   if (P.order1) {
     // the queue that phase 0 filled, ordered by the histories' phase-1 cost
@@ -1107,7 +1106,7 @@ int launch_mc_t(dp_ctx* ctx, McParams& P) {
     --ctx->launches;
     timed_end(ctx, "mc_order");
   }
-  rc = launch_phase<R, 1, T, POR>(ctx, P, smem, need);
+  rc = launch_phase<R, 1, T, POR>(ctx, P, smem);
   if (rc) return rc;
   timed_begin(ctx);
   mc_finish_kernel<R><<<int(rec_blocks), 256, 0, ctx->stream>>>(P);

@@ -129,6 +129,33 @@ __device__ __forceinline__ long next_history(unsigned long long* counter) {
   return long(base + g.thread_rank());
 }
 
+// First hand-out of a launch: the place in the hand-out order of the history that
+// this thread starts with (n or more: none); the counter then deals from
+// deal_first(n) on.  Fewer histories than lanes are spread over all warps of the
+// grid, first one warp of every CTA, then the next, and lanes are filled once every
+// warp has one: a lane alone in its warp costs the FP64 pipe as much as a full warp
+// (64 cycles per instruction, measured) and FP32 little, but a history's divergent
+// paths (hard events, rejection loops) then wait for no other lane.  The places are
+// dealt by warp and not by arrival: longest first, the CTAs that arrive first would
+// hold all the long histories and the other SMs would idle at the end.  FP64,
+// run_backward_mc, 100 m of rock: 10^3 histories 64.7 -> 37.9 ms against full warps
+// on the fewest CTAs (with the steps and sums of that build); dealt by warp and not
+// by arrival, 10^4 36.5 -> 29.7 ms and 5 10^4 through a mixture 85 -> 62 ms.  FP32,
+// the same rock: 10^3 12.5 -> 4.5 ms, 10^4 14.9 -> 6.9, 10^5 16.3 -> 13.4, 4 10^5 26.3
+// -> 26.0 against full warps on the fewest CTAs, dealt by arrival.
+__device__ __forceinline__ long deal_per_warp(long n) {
+  const long warps = long(gridDim.x) * (blockDim.x >> 5);
+  return n >= 32 * warps ? 32 : (n <= warps ? 1 : (n + warps - 1) / warps);
+}
+// (past n where every history has been dealt)
+__device__ __forceinline__ long deal_first() { return long(gridDim.x * blockDim.x); }
+__device__ __forceinline__ long deal_place(long n) {
+  const long l = deal_per_warp(n), w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // every other row of warps runs backwards over the CTAs
+  const long rank = w * gridDim.x + ((w & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+  return lane < l ? rank * l + lane : n;
+}
+
 // A block whose table staging gave up takes its share of the phase's
 // histories all the same and ends each one flagged DP_ST_TABLE_WAIT (no flux,
 // no table read), so that every history of the launch is accounted for.
@@ -139,9 +166,7 @@ __device__ __forceinline__ void drain_histories(G& geo, unsigned long long* coun
   const long n = PHASE == 0 ? geo.n0() : long(*(volatile unsigned long long*)(counter + 2));
   typename G::Hist h;
   Stream g;
-  for (;;) {
-    const long j = next_history(counter + PHASE);
-    if (j >= n) break;
+  for (long j = deal_place(n); j < n; j = deal_first() + next_history(counter + PHASE)) {
     const long k = order ? long(order[j]) : j;
     long i = k;
     if (PHASE == 0) geo.start(k, h, g);
@@ -269,34 +294,6 @@ __device__ __forceinline__ void serve_cta(const G& geo, const Consts& C, float* 
   }
 }
 
-// First hand-out of the FP64 transport: the place in the hand-out order of the
-// history this thread starts with (n or more: none); the counter then deals from
-// fp64_first(n) on.  An FP64 warp instruction holds its SM partition for 64
-// cycles with one lane active as with 32 (measured), so a lane alone in its warp
-// costs as much as a full warp, but a history's divergent paths (hard events,
-// rejection loops) then wait for no other lane.  So the histories are spread over
-// all warps of the grid, first one warp of every CTA, then the next, and lanes
-// are filled once every warp has one.  The places are dealt by warp and not by
-// arrival: longest first, the CTAs that arrive first would hold all the long
-// histories and the other SMs would idle at the end.  run_backward_mc, 100 m of
-// rock: 10^3 histories 64.7 -> 37.9 ms against full warps on the fewest CTAs (with
-// the steps and sums of that build); dealt by warp and not by arrival, 10^4 36.5
-// -> 29.7 ms and 5 10^4 through a mixture 85 -> 62 ms.
-__device__ __forceinline__ long fp64_per_warp(long n) {
-  const long warps = long(gridDim.x) * (blockDim.x >> 5);
-  return n >= 32 * warps ? 32 : (n <= warps ? 1 : (n + warps - 1) / warps);
-}
-__device__ __forceinline__ long fp64_first(long n) {
-  const long first = long(gridDim.x) * (blockDim.x >> 5) * fp64_per_warp(n);
-  return first < n ? first : n;
-}
-__device__ __forceinline__ long fp64_place(long n) {
-  const long l = fp64_per_warp(n), w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // every other row of warps runs backwards over the CTAs
-  const long rank = w * gridDim.x + ((w & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-  return lane < l ? rank * l + lane : n;
-}
-
 // Runs histories until none is left for this phase.  counter[PHASE] hands out
 // history indices, counter[2] counts the hand-off queue.  `coop` is the CTA's
 // shared memory for DCS sums.  FP32: per warp `stride` floats (coop_floats for
@@ -329,8 +326,7 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
     return true;
   };
   auto take = [&](long* idx) -> bool {
-    const long j = next_history(counter + PHASE);
-    return begin(sizeof(R) == 8 ? fp64_first(n) + j : j, idx);
+    return begin(deal_first() + next_history(counter + PHASE), idx);
   };
   // after a step: end the history, hand it to phase 1, or keep going
   auto settle = [&](int r, long* idx) -> bool {
@@ -346,8 +342,8 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
     return true;
   };
   long i = 0;
+  bool live = begin(deal_place(n), &i);
   if constexpr (sizeof(R) == 4) {
-    bool live = take(&i);
     if (lockstep && kc > 0) {
       int* cnt = reinterpret_cast<int*>(coop);
       if (threadIdx.x == 0) cnt[0] = cnt[1] = 0;
@@ -423,7 +419,6 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
     // on the terms of the event's sum (del64_sum)
     const int lane = threadIdx.x & 31;
     double* buf = reinterpret_cast<double*>(coop + size_t(threadIdx.x >> 5) * stride);
-    bool live = begin(fp64_place(n), &i);
     while (__any_sync(0xffffffffu, live)) {
       unsigned want = __ballot_sync(0xffffffffu, live && h.x.kind != CONT_NONE);
       while (want) {
