@@ -434,37 +434,6 @@ struct McParams {
   uint32_t *order0, *order1, *sched;
 };
 
-// Cost buckets of a history for the longest-first schedule.  Phase 0 (below
-// the mode switch): its step count follows log(1 + G / X0), G the rock
-// grammage along the direction and X0 the CSDA range at the start energy
-// (the step limits are a fixed fraction of the range), 64 buckets per unit.
-// Phase 1 (mixed steps from hard event to hard event): it follows the rock
-// grammage left above the switch, log(1 + G1 / 1e4 kg/m^2), 128 buckets per
-// unit.  A history above the switch at the start costs phase 0 nothing.
-template <class R>
-__device__ __forceinline__ void cost_buckets(const Med<R>& rock, const Consts& C, double E0,
-                                             double thick, double rho, double uz, uint16_t* k0,
-                                             uint16_t* k1) {
-  const double G = thick * rho / fmax(fabs(uz), 0.05);
-  const double X0 = double(at(rock, locate(rock, R(E0)), MC_CR));
-  const double Xs = double(at(rock, locate(rock, R(C.thr_low)), MC_CR));
-  const double G1 = fmax(G - fmax(Xs - X0, 0.0), 0.0);
-  const double c0 = E0 < C.thr_low ? log1p(G / fmax(X0, 1e-3)) * 64.0 : 0.0;
-  const double c1 = log1p(G1 * 1e-4) * 128.0;
-  *k0 = uint16_t(fmin(c0, double(kSchedBuckets - 1)));
-  *k1 = uint16_t(fmin(c1, double(kSchedBuckets - 1)));
-}
-struct KeyOf {
-  const uint16_t* key;
-  __device__ int operator()(long s) const { return key[s]; }
-};
-template <class Q>
-struct QueueKeyOf {
-  const Q* queue;
-  const uint16_t* key;
-  __device__ int operator()(long s) const { return key[queue[s].index]; }
-};
-
 // Start record of history i: energy, charge and weight drawn as
 // run_backward_mc draws them (src/Geometry.jl:863-875) or given; geometry
 // given, taken from its line of sight or drawn (Philox blocks 1-2).
@@ -521,7 +490,7 @@ __global__ void __launch_bounds__(256) mc_init_kernel(const __grid_constant__ Mc
     double theta = (90.0 - elev) * kPi / 180.0;
     if (P.key0) {
       const Med<R> rock = make_med<R>(P.blob, P.lay, P.info[0]);
-      cost_buckets<R>(rock, P.C, E0, thick, rho, cos(theta), P.key0 + i, P.key1 + i);
+      cost_buckets<R>(rock, P.C, E0, thick * rho / fmax(fabs(cos(theta)), 0.05), P.key0 + i, P.key1 + i);
     }
     StartRec<R> r;
     r.thick = alt_make<R>(thick);
@@ -878,24 +847,6 @@ namespace {
 // Per-history device records of a run (hand-off, start, end), sized for FP64.
 constexpr size_t kRecBytes = sizeof(HandoffP<double>) + sizeof(StartRec<double>) +
                              sizeof(EndRec<double>) + sizeof(PorousRec<double>) + 64;
-// The longest-first schedule: two cost buckets and two order entries per
-// history, and the counting-sort words (kSchedExtra covers those and the
-// arena's alignment of the five arrays).
-constexpr size_t kSchedBytes = 2 * sizeof(uint16_t) + 2 * sizeof(uint32_t);
-constexpr size_t kSchedExtra = 2 * kSchedBuckets * sizeof(uint32_t) + 5 * 256;
-
-// Takes the schedule's arrays from the arena when the context hands
-// histories out longest first (and the indices fit 32 bits).
-void take_sched(dp_ctx* ctx, int precision, long n, Arena& A, McParams& P) {
-  if (ctx->mc_order[DP_KERNEL_MC][precision] != 0 || n >= (1L << 32)) return;
-  P.key0 = A.take<uint16_t>(n);
-  P.key1 = A.take<uint16_t>(n);
-  P.order0 = A.take<uint32_t>(n);
-  P.order1 = A.take<uint32_t>(n);
-  P.sched = A.take<uint32_t>(2 * kSchedBuckets);
-  if (!P.sched) P.key0 = P.key1 = nullptr, P.order0 = P.order1 = P.sched = nullptr;
-}
-
 }  // namespace
 
 namespace dp {
@@ -1435,7 +1386,7 @@ int dp_mc_histories(dp_ctx* ctx, const dp_physics* ph, const dp_mixture* rock_c,
   P.queue = queue;
   P.start = srec;
   P.end = erec;
-  take_sched(ctx, cfg->precision, n, A, P);
+  take_sched(ctx, DP_KERNEL_MC, cfg->precision, n, A, P);
   rc = run(ctx, P, cfg->precision);
   if (rc) return rc;
   std::vector<int32_t> st_h;
@@ -1587,7 +1538,7 @@ int dp_mc_run_los(dp_ctx* ctx, const dp_physics* ph, dp_mixture* rock, const dp_
       P.info[2] = make_info(porous);
       P.porous_rec = prec;
     }
-    take_sched(ctx, cfg->precision, total, A, P);
+    take_sched(ctx, DP_KERNEL_MC, cfg->precision, total, A, P);
     rc = run(ctx, P, cfg->precision);
     if (rc) return rc;
     if (compute_gradient) {

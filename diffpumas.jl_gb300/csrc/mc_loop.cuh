@@ -543,5 +543,54 @@ inline cudaError_t sched_order(cudaStream_t st, long n, const unsigned long long
   return cudaGetLastError();
 }
 
+// Cost buckets of a history for the longest-first schedule.  Phase 0 (below
+// the mode switch): its step count follows log(1 + G / X0), G the rock
+// grammage (kg/m^2) along the direction and X0 the CSDA range at the start energy
+// (the step limits are a fixed fraction of the range), 64 buckets per unit.
+// Phase 1 (mixed steps from hard event to hard event): it follows the rock
+// grammage left above the switch, log(1 + G1 / 1e4 kg/m^2), 128 buckets per
+// unit.  A history above the switch at the start costs phase 0 nothing.
+template <class R>
+__device__ __forceinline__ void cost_buckets(const Med<R>& rock, const Consts& C, double E0, double G,
+                                             uint16_t* k0, uint16_t* k1) {
+  const float X0 = float(at(rock, locate(rock, R(E0)), MC_CR));
+  const float Xs = float(at(rock, locate(rock, R(C.thr_low)), MC_CR));
+  const float g = float(G), g1 = fmaxf(g - fmaxf(Xs - X0, 0.f), 0.f);
+  const float c0 = E0 < C.thr_low ? log1pf(g / fmaxf(X0, 1e-3f)) * 64.f : 0.f;
+  const float c1 = log1pf(g1 * 1e-4f) * 128.f;
+  *k0 = uint16_t(fmaxf(fminf(c0, float(kSchedBuckets - 1)), 0.f));
+  *k1 = uint16_t(fmaxf(fminf(c1, float(kSchedBuckets - 1)), 0.f));
+}
+struct KeyOf {
+  const uint16_t* key;
+  __device__ int operator()(long s) const { return key[s]; }
+};
+template <class Q>
+struct QueueKeyOf {
+  const Q* queue;
+  const uint16_t* key;
+  __device__ int operator()(long s) const { return key[queue[s].index]; }
+};
+
+// The longest-first schedule: two cost buckets and two order entries per
+// history, and the counting-sort words (kSchedExtra covers those and the
+// arena's alignment of the five arrays).
+constexpr size_t kSchedBytes = 2 * sizeof(uint16_t) + 2 * sizeof(uint32_t);
+constexpr size_t kSchedExtra = 2 * kSchedBuckets * sizeof(uint32_t) + 5 * 256;
+
+// Takes the schedule's arrays from the arena when the context hands
+// histories out longest first (and the indices fit 32 bits).
+template <class P>
+inline void take_sched(dp_ctx* ctx, int family, int precision, long n, Arena& A, P& p) {
+  if (ctx->mc_order[family][precision] != 0 || n >= (1L << 32)) return;
+  p.key0 = A.take<uint16_t>(n);
+  p.key1 = A.take<uint16_t>(n);
+  p.order0 = A.take<uint32_t>(n);
+  p.order1 = A.take<uint32_t>(n);
+  p.sched = A.take<uint32_t>(2 * kSchedBuckets);
+  if (!p.sched) p.key0 = p.key1 = nullptr, p.order0 = p.order1 = p.sched = nullptr;
+}
+
+
 }  // namespace mc
 }  // namespace dp

@@ -1,7 +1,8 @@
 """How the stochastic kernels deal histories to their lanes: counts around one per
-multiprocessor, one per warp, two per warp and all lanes, both precisions.  A
-history draws from its own stream and its sums do not depend on the histories beside
-it, so a run's histories are bitwise the first ones of a longer run."""
+multiprocessor, one per warp, two per warp and all lanes, both precisions, longest
+first and in index order.  A history draws from its own stream and its sums do not
+depend on the histories beside it, so a run's histories are bitwise the first ones
+of a longer run, and the order changes nothing."""
 import numpy as np
 import pytest
 
@@ -38,3 +39,26 @@ def test_histories_do_not_depend_on_their_number(setting, precision):
     for n in counts:
         for a, b in zip(run(n), ref):
             np.testing.assert_array_equal(a, b[:n])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [1, 153, 700, 6000])
+def test_directions_do_not_depend_on_the_order(setting, precision, n):
+    dp, phys = setting
+    wf = np.linspace(0.0, 0.5, 9)
+    cfg, site = dp.MaterialConfig(1, 3, 2, -1, 2650.0, 1000.0, 0.0, 0.0), dp.SiteConfig(963.0, 2000.0)
+    seg = lambda *c: [dp.CellSegment(k, 1.5 * k) for k in c]  # noqa: E731
+    P = dp.DirectionalPath
+    paths = [P(0.0, 0.0, [], 0.0, 0.0, 0.0, 0.0, True), P(10.0, 0.0, seg(1, 2), 0.0, 0.0, 6.0, 50.0, True),
+             P(30.0, 0.0, seg(2, 3), 0.0, 0.0, 1.0, 30.0, False), P(60.0, 0.0, seg(*range(1, 10)), 0.0, 0.0, 0.0, 90.0, True)]
+    mats, dens = dp.build_cell_properties_for_mc(phys, np.zeros(9, bool), wf, cfg)
+    batch = dp.DirBatch(phys, cfg, site, paths, mats, dens, None, n_samples=n, energy_min=0.1, energy_max=1e4)
+    out, before = [], dp.get_mc_shape(phys.ctx, "dir", precision)
+    try:
+        for order in (0, 1):
+            dp.set_mc_shape(phys.ctx, "dir", precision, order=order)
+            out.append(batch.run(5, precision=precision, return_histories=True))
+    finally:
+        dp.set_mc_shape(phys.ctx, "dir", precision, order=before["order"])
+    for k in out[0]:
+        np.testing.assert_array_equal(out[0][k], out[1][k])
