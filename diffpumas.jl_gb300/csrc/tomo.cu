@@ -491,6 +491,14 @@ __device__ __forceinline__ float gccly32(float cs, float cs129, float K, float q
   return f;
 }
 
+// a / b for b inside the normal range, y = __frcp_rn(b): the rounded quotient
+// (f64::div_rn's method) as long as its remainder does not underflow.
+__device__ __forceinline__ float div32(float a, float b, float y) {
+  float q = a * y;
+  q = fmaf(fmaf(-b, q, a), y, q);
+  return fmaf(fmaf(-b, q, a), y, q);
+}
+
 // Float-pair accumulation (TwoSum): (h, l) += x
 __device__ __forceinline__ void ff_add(float& h, float& l, float x) {
   float s = h + x;
@@ -539,7 +547,7 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
   __syncthreads();
   const float inv_m = float(1.0 / P.mass), inv_ctau = float(1.0 / P.ctau);
   const float Lair_c = float(P.H - P.zmax), Gair_c = float(1.205 * 12e3 * P.air_dexp);
-  const float m_ctau = float(P.mass * P.ctau);
+  const float m_ctau = float(P.mass * P.ctau), i_m_ctau = __frcp_rn(m_ctau);
   const float Emax = EE[n - 1];
   for (long q = blockIdx.x * long(kWarps) + warp; q < P.n_rays; q += long(gridDim.x) * kWarps) {
     const long r = P.order[q];
@@ -615,7 +623,8 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
         float Ek = EN;
         int ik = iN;
         bool ck = clampN;
-        for (int s = nseg - 1; s >= 0; --s) {
+        // the cotangent of one segment's density for this lane's node
+        auto back = [&](int s) {
           // previous point E_{k-1}
           ff_add(yh, yl, -sG[s]);
           float Ekm1;
@@ -636,16 +645,37 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
           const float Kp = ck ? 0.0f : Ek * SLO[ik];
           const float x = 0.5f * (Ekm1 + Ek) * inv_m;
           const float ib = rsqrtf(x * (x + 2.0f));
-          const float a = sL[s] * (x + 1.0f) * ib * ib * ib / m_ctau;
+          const float a = div32(sL[s] * (x + 1.0f) * ib * ib * ib, m_ctau, i_m_ctau);
           lam += 0.5f * a;
-          float v = cf * lam * Kp * sL[s];
+          const float v = cf * lam * Kp * sL[s];
           const float Rp = cm ? 0.0f : 1.0f / (Ekm1 * SLO[im]);
           lam = lam * Kp * Rp + 0.5f * a;
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) sJ[s] += v;
           Ek = Ekm1;
           ik = im;
           ck = cm;
+          return v;
+        };
+        // Sums over the warp's nodes, four segments at a time: the butterfly of one
+        // segment with the halves and quarters of the warp on different segments,
+        // so 6 exchanges for four sums instead of 20, the same additions.  The
+        // kernel is bound by the instructions it issues (80% of its cycles): 6.5 10^6
+        // segments, 32 nodes, with the gradient 1.72 -> 1.49 ms by this and div32.
+        int s = nseg - 1;
+        for (; s >= 3; s -= 4) {
+          const float v0 = back(s), v1 = back(s - 1), v2 = back(s - 2), v3 = back(s - 3);
+          const bool h = lane & 16, g = lane & 8;
+          float a = h ? v1 : v0, b = h ? v3 : v2;
+          a += __shfl_xor_sync(0xffffffffu, h ? v0 : v1, 16);
+          b += __shfl_xor_sync(0xffffffffu, h ? v2 : v3, 16);
+          float v = g ? b : a;
+          v += __shfl_xor_sync(0xffffffffu, g ? a : b, 8);
+          for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if ((lane & 7) == 0) sJ[s - (h ? 1 : 0) - (g ? 2 : 0)] += v;
+        }
+        for (; s >= 0; --s) {
+          float v = back(s);
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0) sJ[s] += v;
         }
       }
     }
