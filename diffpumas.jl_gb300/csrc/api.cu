@@ -235,13 +235,13 @@ static int finish_upload(dp_ctx* ctx, dp_physics* p, dp_physics** out) {
   }
   // single-precision derived columns
   p->ld32 = dp::padded32(p->n);
-  std::vector<float> t32(size_t(p->n_mat) * dp::kNC32 * p->ld32, 0.0f);
+  std::vector<float> t32(size_t(p->n_mat) * dp::kNC32Rows * p->ld32, 0.0f);
   for (int m = 0; m < p->n_mat; ++m) {
     const double* E = &p->host[(size_t(m) * DP_NCOL + DP_COL_E) * p->n];
     const double* L = &p->host[(size_t(m) * DP_NCOL + DP_COL_LOGE) * p->n];
     const double* R = &p->host[(size_t(m) * DP_NCOL + DP_COL_CSDA_R) * p->n];
     const double* S = &p->host[(size_t(m) * DP_NCOL + DP_COL_CSDA_S) * p->n];
-    auto C = [&](int c) { return &t32[(size_t(m) * dp::kNC32 + c) * p->ld32]; };
+    auto C = [&](int c) { return &t32[(size_t(m) * dp::kNC32Rows + c) * p->ld32]; };
     for (int i = 0; i < p->n; ++i) {
       float rh = float(R[i]);
       C(dp::C32_RH)[i] = rh;
@@ -255,6 +255,17 @@ static int finish_upload(dp_ctx* ctx, dp_physics* p, dp_physics** out) {
         C(dp::C32_DSDLE)[i] = float((S[i + 1] - S[i]) / dl);
         C(dp::C32_DLE)[i] = float(dl);
       }
+    }
+    for (int i = 0; i < p->n; ++i) {
+      float *a = C(dp::kNC32) + 4 * i, *b = C(dp::kNC32 + 4) + 4 * i;
+      a[0] = C(dp::C32_RH)[i];
+      a[1] = C(dp::C32_RH)[i + 1 < p->n ? i + 1 : i];
+      a[2] = C(dp::C32_SLOPE)[i];
+      a[3] = C(dp::C32_DLE)[i];
+      b[0] = C(dp::C32_RL)[i];
+      b[1] = C(dp::C32_E)[i];
+      b[2] = C(dp::C32_S)[i];
+      b[3] = C(dp::C32_DSDLE)[i];
     }
   }
   if (cudaMalloc(&p->dev32, t32.size() * sizeof(float)) != cudaSuccess ||

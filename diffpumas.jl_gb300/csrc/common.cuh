@@ -53,6 +53,9 @@ struct TabView {
 //   DSDLE    (S[i+1]-S[i]) / (logE[i+1]-logE[i])     (d S / d log E)
 //   DLE      logE[i+1]-logE[i]
 enum Col32 { C32_RH = 0, C32_RL, C32_S, C32_E, C32_LE, C32_SLOPE, C32_DSDLE, C32_DLE, kNC32 };
+// The columns of a material are followed by as many words in rows, four per node:
+// first {RH of i, RH of i + 1, SLOPE, DLE}, then {RL, E, S, DSDLE}.
+constexpr int kNC32Rows = 2 * kNC32;  // words per node and material
 DP_HD int padded32(int n) { return (n + 3) & ~3; }
 
 // ------------------------------------------------------------- dual numbers

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(128) csda32_kernel(CsdaParams P, const float* 
   for (int m = 0; m < 2; ++m)
     for (int c = 0; c < F_NCOL; ++c)
       src[m * F_NCOL + c] = reinterpret_cast<const double*>(
-          tab32 + (size_t(m == 0 ? P.rock : P.air) * kNC32 + cols[c]) * ld32);
+          tab32 + (size_t(m == 0 ? P.rock : P.air) * kNC32Rows + cols[c]) * ld32);
   if (!stage_columns(smem, src, 2 * F_NCOL, uint32_t(ld32 * sizeof(float)), &mbar, P.wait_iters)) {
     if (threadIdx.x == 0) atomicExch(P.err_flag, 1);
     return;

@@ -149,7 +149,7 @@ struct dp_physics {
   double* dev = nullptr;              // n_mat x DP_NCOL x ld
   dp::TabView view{};
   // Single-precision derived columns for the mixed-precision kernels:
-  // n_mat x dp::kNC32 x ld32 floats (see dp::Col32).
+  // n_mat x dp::kNC32Rows x ld32 floats (see dp::Col32).
   float* dev32 = nullptr;
   int ld32 = 0;
 };
