@@ -16,15 +16,14 @@
 // X = R(E), E' = R^-1(X + rho L), weight *= S(E')/S(E) * exp(-L/(beta gamma
 // c tau)); then the closed-form air column and the GCCLY flux; the per-ray
 // flux is (1/N) sum_n 2 w_n f_n (compute_flux_from_segments, :374-470).
-//  * FP64 kernel: the reference's per-segment operations (parity mode).
+//  * FP64 kernel (tomo_fp64.cuh): the same program in FP64 (parity mode).
 //  * Mixed kernel: per-segment work in FP32 -- the range is carried as a float
 //    pair (the inversion stays accurate near E_min), energies come from the
 //    node energy times exp of a small log offset, stopping powers and decay
 //    exponents in FP32; the node flux integral is accumulated in FP64.
 // Adjoint: a reverse sweep over the segment list carries
 // lambda_k = d log(flux)/d E_k; d flux/d rho_k = flux lambda_k dE_k/dY_k L_k.
-// Lanes are reduced per segment by a fixed shuffle tree: one Jacobian entry per
-// segment.  J^T r = per-cell sums over the precomputed CSC permutation, each
+// Lanes are reduced per segment by a fixed tree: one Jacobian entry per segment.  J^T r = per-cell sums over the precomputed CSC permutation, each
 // bucket ordered by entry index -- no floating-point atomics, bitwise
 // reproducible.
 #include <math_constants.h>
@@ -447,13 +446,27 @@ constexpr int kWarps = 4;
 #include "tomo_fp64.cuh"
 
 // ---------------------------------------------------------------- mixed kernel
-// Node start from the FP64 tables (each block computes all nodes once).
+// Node start from the FP64 tables, computed by each block for itself: one logarithm,
+// one division and two interpolations in place of two dual-number lookups.  4096
+// rays, flux only, 32 nodes: 76 -> 69 us; 8000 rays with the gradient, 70 nodes: 297 ->
+// 285 us.
 __device__ __forceinline__ void node_init(const EvalP& P, int k, const float4* RA, NodeInit* out) {
   const double E0 = P.nE[k];
-  const Dd lE = dd(log(E0));
   const double *E = P.tab.col(0, DP_COL_E), *LE = P.tab.col(0, DP_COL_LOGE);
-  const double X0 = interp_logE(P.tab, E, LE, P.tab.col(P.rock, DP_COL_CSDA_R), dd(E0), lE, nullptr).v;
-  const double S0 = interp_logE(P.tab, E, LE, P.tab.col(P.rock, DP_COL_CSDA_S), dd(E0), lE, nullptr).v;
+  const double *R = P.tab.col(P.rock, DP_COL_CSDA_R), *S = P.tab.col(P.rock, DP_COL_CSDA_S);
+  const int last = P.tab.n - 1;
+  double X0, S0;  // linear in log E (src/Physics.jl:660-687)
+  if (E0 <= E[0] || E0 >= E[last]) {
+    X0 = R[E0 <= E[0] ? 0 : last];
+    S0 = S[E0 <= E[0] ? 0 : last];
+  } else {
+    const double lE = f64::log(E0);
+    const int i = P.tab.uniform ? uniform_interval(LE, last + 1, lE, P.tab.lE0, P.tab.inv_dlE)
+                                : bisect(LE, last + 1, lE);
+    const double t = f64::div(lE - LE[i], LE[i + 1] - LE[i]);
+    X0 = fma(t, R[i + 1] - R[i], R[i]);
+    S0 = fma(t, S[i + 1] - S[i], S[i]);
+  }
   NodeInit o;
   o.yh = float(X0);
   o.yl = float(X0 - double(o.yh));

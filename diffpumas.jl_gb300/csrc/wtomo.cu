@@ -2,8 +2,8 @@
 // the device: compute_directional_flux_csda (:667-727),
 // directional_flux_and_grad_csda and assemble_forward_and_jacobian
 // (:736-820), with the CSDA correction multipliers (:85-214, :367-412,
-// :557-579).  Two instances of the walk: FP64 (wtomo_fp64.cuh), the
-// reference's operations, and mixed precision (wtomo_walk.cuh), FP32 steps and tangents with
+// :557-579).  Two instances of the walk: FP64 (wtomo_fp64.cuh) and
+// mixed precision (wtomo_walk.cuh), FP32 steps and tangents with
 // the adjoint's prefix sums, the flux and the reductions in FP64.
 //
 // One warp per direction, one lane per energy sample.  d flux / d w comes from
