@@ -118,6 +118,23 @@ __device__ __forceinline__ bool lt_pos(double a, double b) {
 __device__ __forceinline__ double min_pos(double a, double b) { return lt_pos(b, a) ? b : a; }
 __device__ __forceinline__ double max_pos(double a, double b) { return lt_pos(a, b) ? b : a; }
 
+// Offset of lx, in widths, on the interval of the increasing grid x that it lies
+// in: (lx - x[i]) inv[i] (inv: inverse widths), searched from interval i, which
+// becomes that interval.  The searches decide by the sign and the exponent of the
+// offset, which the caller wants anyway: no FP64 comparison.  One way only: beside
+// a node the rounded offsets of both its intervals can point at the other one (a
+// last place below a node near 0 is below 0 on the one and rounds to 1 on the
+// other), and either then stands for the node.
+__device__ __forceinline__ double grid_offset(const double* x, const double* inv, int n, double lx, int& i) {
+  for (int way = 0;;) {
+    const double t = (lx - x[i]) * inv[i];
+    const int h = hi32(t), step = h < 0 && i > 0 ? -1 : (h >= 0x3ff00000 && i < n - 2 ? 1 : 0);
+    if (step == 0 || step == -way) return t;
+    way = step;
+    i += step;
+  }
+}
+
 // u01 on the bit pattern: m 2^-53 of the 53-bit integer m, no FP64 instruction.
 __device__ __forceinline__ double uniform(uint32_t a, uint32_t b) {
   const uint64_t m = (uint64_t(a >> 5) << 26) | uint64_t(b >> 6);

@@ -52,14 +52,9 @@ __device__ __forceinline__ Loc<double> locate_log(const Med<double>& m, double x
   } else {
     i = bisect_r(lE, m.n, lx);
   }
-  for (;;) {
-    L.i = i;
-    L.t = (lx - lE[i]) * inv[i];
-    const int h = f64::hi32(L.t);
-    const int move = h < 0 && i > 0 ? -1 : (h >= 0x3ff00000 && i < m.n - 2 ? 1 : 0);
-    if (move == 0) return L;
-    i += move;
-  }
+  L.t = f64::grid_offset(lE, inv, m.n, lx, i);
+  L.i = i;
+  return L;
 }
 __device__ __forceinline__ Loc<double> locate(const Med<double>& m, double x) {
   return locate_log(m, x, log64(x));

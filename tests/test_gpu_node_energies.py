@@ -1,0 +1,43 @@
+"""Histories and samples that start exactly on nodes of the energy grid (the ordinary
+input of a scan over tabulated energies), on grids where the device's logarithm of
+such an energy and the table's differ by a last place, against the oracle.
+
+A node has the same energy in both its intervals, so nothing is gained or lost there: the
+tolerances are those of the other FP64 comparisons of each model."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# grids with such a node near 1 GeV (0.9659 and 0.9771 GeV), and a coarser one
+GRIDS = [(200, 1e-3, 1e8), (200, 1e-3, 1e4), (80, 1e-3, 1e6)]
+
+
+@pytest.fixture(scope="module", params=GRIDS, ids=["1e8", "1e4", "80"])
+def setting(request, oracle):
+    import dpgpu as dp
+    n, lo, hi = request.param
+    orc = oracle.default_physics((oracle.STANDARD_ROCK, oracle.AIR, oracle.WATER), n=n, Kmin=lo, Kmax=hi, coulomb=True)
+    phys = dp.upload_physics([orc.table(i) for i in range(3)], ["StandardRock", "Air", "Water"],
+                             materials=(dp.STANDARD_ROCK, dp.AIR, dp.WATER))
+    E = np.asarray(orc.column(0, "E"), float)
+    return dp, orc, phys, E[(E > 0.05) & (E < 100.0)]
+
+
+def test_histories(setting, oracle):
+    """As the other histories: 1e-9, and rounding flips a decision in under 1 %."""
+    dp, orc, phys, nodes = setting
+    E = np.tile(nodes, 1 + 1000 // len(nodes))
+    n = len(E)
+    rng = np.random.default_rng(1)
+    q, w = np.where(rng.random(n) > 0.5, 1.0, -1.0), 2.0 * E
+    rock, air = dp.MaterialMixture(phys, 1), dp.MaterialMixture(phys, 2)
+    geo = dict(thickness=rng.uniform(1.0, 30.0, n), density=rng.uniform(2000.0, 2800.0, n),
+               elevation=rng.uniform(30.0, 90.0, n), primary_altitude=np.full(n, 1300.0))
+    c, st, steps, Ef = dp.mc_histories(phys, rock, air, E, q, w, seed=5, precision="fp64", **geo)
+    oc, ost, osteps, oE = oracle.mc_histories(orc, [0], 1, geo["thickness"], geo["density"], geo["elevation"],
+                                              geo["primary_altitude"], E, q, w, seed=5)
+    assert (st == 0).all() and (ost == 0).all()
+    near = lambda a, b: np.abs(a - b) <= 1e-9 * np.maximum(np.abs(a), np.abs(b)) + 1e-300  # noqa: E731
+    same = near(c, oc) & (steps == osteps) & near(Ef[:, 0], oE)
+    assert (~same).sum() <= 0.01 * n, (~same).sum()
