@@ -59,15 +59,10 @@ __device__ __forceinline__ Pos locate(const Tables& tb, double E, int i) {
     p = Pos{tb.n - 2, 1.0, 0.0};
   } else if (b > tb.lo) {
     const double lE = f64::log(E);
-    const double* lx = tb.c[wt::S_LE];
     const double* inv = tb.d[D_INV];
-    for (;;) {
-      p = Pos{i, (lE - lx[i]) * inv[i], inv[i]};
-      const int h = f64::hi32(p.t);  // 0 <= t < 1, or an end interval
-      const int step = h >= 0x3ff00000 && i < tb.n - 2 ? 1 : (h < 0 && i > 0 ? -1 : 0);
-      if (step == 0) break;
-      i += step;
-    }
+    p.t = f64::grid_offset(tb.c[wt::S_LE], inv, tb.n, lE, i);
+    p.i = i;
+    p.il = inv[i];
   }
   __syncwarp();
   return p;

@@ -41,3 +41,23 @@ def test_histories(setting, oracle):
     near = lambda a, b: np.abs(a - b) <= 1e-9 * np.maximum(np.abs(a), np.abs(b)) + 1e-300  # noqa: E731
     same = near(c, oc) & (steps == osteps) & near(Ef[:, 0], oE)
     assert (~same).sum() <= 0.01 * n, (~same).sum()
+
+
+def test_water_fraction_samples(setting, oracle):
+    """As the other FP64 walks: 1e-10 on the flux, 1e-8 on the Jacobian.  The first
+    sample of every path starts on its node with no step before it."""
+    from test_gpu_wtomo import _oracle, _per_cell_first
+    dp, orc, phys, nodes = setting
+    rng = np.random.default_rng(3)
+    wf = rng.uniform(0.0, 0.9, 9)
+    seg = lambda *c: [dp.CellSegment(int(k), float(rng.uniform(1e-3, 60.0))) for k in c]  # noqa: E731
+    P = dp.DirectionalPath
+    paths = [P(0.0, 0.0, [], 0.0, 0.0, 0.0, 0.0, True), P(10.0, 0.0, [], 0.0, 0.0, 120.0, 50.0, True),
+             P(60.0, 0.0, seg(*range(1, 10)), 0.0, 0.0, 5.0, 500.0, True)]
+    cfg, site = dp.MaterialConfig(1, 3, 2, -1, 2650.0, 1000.0, 0.0, 0.0), dp.SiteConfig(963.0, 3e4)
+    E = nodes[:256]
+    samples = [dp.EnergySample(float(e), 1.0 if k % 2 else -1.0, 0.1 * float(e)) for k, e in enumerate(E)]
+    f, seg_ptr, cells, jac = dp.csda_flux_batch(phys, np.zeros(9, bool), cfg, site, paths, wf, samples)
+    of, og = _oracle(oracle, orc, wf, paths, samples, [0] * 10)
+    np.testing.assert_allclose(f, of, rtol=1e-10, atol=0)
+    np.testing.assert_allclose(_per_cell_first(seg_ptr, cells, jac), og, rtol=1e-8, atol=1e-12 * np.abs(og).max())
