@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
     double fsum = 0.0;
     for (int base = 0; base < P.n_nodes; base += 32) {
       const int nd = base + lane;
-      const bool active = nd < P.n_nodes;
+      // (a NaN node energy ends its node at the first segment: it takes no part)
+      const bool active = nd < P.n_nodes && !(nseg > 0 && is_nan_bits(P.nE[nd]));
       const double E0 = active ? P.nE[nd] : 1.0;
       // the node's place: interval i, offset t in log E; edge: clamped there
       int i = 0;
@@ -99,7 +100,9 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
       for (int s = 0; s < nseg; ++s) {
         const double L = sL[s], Yn = Y + sG[s];
         double En;
-        if (!f64::lt_pos(Yn, Rhi)) {  // past the table (a NaN density too)
+        // clamped at a table end; a NaN (of either sign: the comparisons are of bits)
+        // arrives at one of them too and ends the node
+        if (!f64::lt_pos(Yn, Rhi)) {
           ok = ok && !is_nan_bits(Yn);
           i = n - 2;
           t = 1.0;
@@ -108,6 +111,7 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
           K = 0.0;
           edge = true;
         } else if (!f64::lt_pos(Rlo, Yn)) {
+          ok = ok && !is_nan_bits(Yn);
           i = 0;
           t = 0.0;
           Y = Rlo;
