@@ -205,6 +205,14 @@ template <int N, class M>
 __device__ __forceinline__ void solid_segment(const Tables& tb, const Run& R, const M& m, double rho,
                                               double irho, double lrho, double distance, Walk<N>& k,
                                               double& ratio, double& tau, double (&g)[N], bool& ok) {
+  if (!(distance > 1e-8)) {  // no step (the same for the whole warp): nothing of the cell enters
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      k.dE[n] = n == 0 ? 1.0 : 0.0;
+      g[n] = 0.0;
+    }
+    return;
+  }
   begin(tb, m, k);
   const double iS0 = f64::rcp(k.S);
   double g0[N], drem[N];
