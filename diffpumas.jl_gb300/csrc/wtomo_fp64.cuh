@@ -130,7 +130,7 @@ __device__ __forceinline__ void begin(const Tables& tb, const M& m, Walk<N>& k) 
   const Pos p = locate(tb, k.E, k.i);
   const Val v = m.at(p);
   k.i = p.i;
-  k.iE = f64::rcp(k.E);
+  k.iE = f64::lt_pos(0.0, k.E) ? f64::rcp(k.E) : 0.0;  // (below the grid no derivative uses it)
   k.S = v.v;
   k.tau = 0.0;
 #pragma unroll

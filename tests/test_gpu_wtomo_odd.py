@@ -1,8 +1,9 @@
 """Odd input of the FP64 water-fraction walk: segments too short for a step (up to 1e-8 m,
-or a NaN length on resident arrays) leave the flux alone whatever their cell holds."""
+or a NaN length on resident arrays) leave the flux alone whatever their cell holds, and
+an energy sample of zero walks from below the grid, where no derivative uses it."""
 import numpy as np
 import pytest
-from test_gpu_wtomo import _samples, dp, orc_phys, phys  # noqa: F401
+from test_gpu_wtomo import _oracle, _per_cell_first, _samples, dp, orc_phys, phys  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +25,19 @@ def test_segments_without_a_step(dp, phys, w, resident):  # noqa: F811
     flux, _ = b.run(np.array([0.1, 0.2, 0.0, 0.0, w]))
     assert flux[0] > 0
     np.testing.assert_array_equal(flux, np.full(len(flux), flux[0]))
+
+
+def test_sample_of_zero_energy(dp, phys, oracle, orc_phys):  # noqa: F811
+    """1e-10 on the flux, 1e-8 on the Jacobian, as the other FP64 walks."""
+    samples = [dp.EnergySample(0.0, 1.0, 1.0), dp.EnergySample(3.0, -1.0, 1.0)]
+    b = _batch(dp, phys, samples, [12.0])
+    wf = np.array([0.1, 0.2, 0.0, 0.0, 0.6])
+    segs = b.arrays["seg_ptr"]
+    flux, jac = b.run(wf)
+    paths = [dp.DirectionalPath(30.0, 0.0, [dp.CellSegment(int(b.arrays["seg_cell"][k]) + 1, float(b.arrays["seg_length"][k]))
+                                            for k in range(segs[i], segs[i + 1])], 0.0, 0.0, 4.0, 60.0, True) for i in range(2)]
+    of, og = _oracle(oracle, orc_phys, wf, paths, samples, [0] * 10)
+    assert np.isfinite(og).all() and (of > 0).all()
+    np.testing.assert_allclose(flux, of, rtol=1e-10, atol=0)
+    g = _per_cell_first(segs, b.arrays["seg_cell"], jac)
+    np.testing.assert_allclose(g, og, rtol=1e-8, atol=1e-12 * np.abs(og).max())
