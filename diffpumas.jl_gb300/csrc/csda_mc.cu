@@ -139,6 +139,8 @@ __device__ __forceinline__ int f_interval(const float* LE, int n, float lx, cons
 //  - a material entered mid-walk is located by the interval and offset the
 //    walk already holds (all materials share the energy grid).
 constexpr int kCsda32Cols = 2 * kNC32 + 1;
+// Dynamic shared memory of a launch that asks for no more (48 KB less the barrier)
+constexpr size_t kSmemDefault = 48 * 1024 - 64;
 __global__ void __launch_bounds__(128, 6) csda32_kernel(CsdaParams P, const float* tab32, int ld32) {
   extern __shared__ __align__(16) double smem[];
   __shared__ uint64_t mbar;
@@ -497,6 +499,9 @@ static int launch(dp_ctx* ctx, CsdaParams& P, const dp_physics* ph32 = nullptr) 
   const size_t smem = ph32 ? size_t(kCsda32Cols) * ph32->ld32 * sizeof(float)
                            : size_t(S_NCOL + D_NCOL) * P.tab.ld * sizeof(double);
   int per_sm = 0, n_sm = 0;
+  // (grids of more than 720 nodes)
+  if (ph32 && smem > kSmemDefault)
+    DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(csda32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   if (ph32)
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csda32_kernel, threads,
                                                                      smem));
