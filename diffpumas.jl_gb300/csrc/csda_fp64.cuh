@@ -51,7 +51,7 @@ struct CsdaConst {
 
 // Geometry of a history as its steps use it.
 struct CsdaWalk {
-  double thick, rho, top;  // top: H - eps
+  double thick, rho, top, rock_top;  // top: H - eps; rock_top: the rock ends there or at H
   double H, uz, inv_uz, air_limit;
   double c, cd, irho;      // rock step limit per range and its tangent, 1 / rho
 };
@@ -61,6 +61,7 @@ __device__ __forceinline__ CsdaWalk csda_walk(double thick, double rho, double H
   w.rho = rho;
   w.H = H;
   w.top = H - kEps64;
+  w.rock_top = w.top < thick ? w.top : thick;
   w.uz = uz;
   w.air_limit = air_limit;
   w.inv_uz = uz > kEps64 || uz < -kEps64 ? 1.0 / uz : 0.0;
@@ -368,7 +369,7 @@ __device__ __forceinline__ int csda_commit(const CsdaTables& T, const CsdaConst&
 // Whether a step of length s at altitude z is cut by nothing but its limit.
 __device__ __forceinline__ bool csda_free(const CsdaWalk& W, bool air, double z, double s) {
   return s < csda_ahead(W, air, z) + 1e-7 && s >= kStepMin && s <= 1000.0 && z >= (air ? W.thick : 0.0) &&
-         z < (air ? W.top : W.thick);
+         z < (air ? W.top : W.rock_top);
 }
 
 __global__ void __launch_bounds__(kCsdaThreads) csda_warp_kernel(CsdaParams P, int group) {
