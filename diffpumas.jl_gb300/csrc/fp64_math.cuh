@@ -146,7 +146,8 @@ __device__ __forceinline__ double uniform(uint32_t a, uint32_t b) {
 // 1 / (beta gamma) at the kinetic energy x (in masses), beta >= 1e-6, and its
 // derivative in x (src/Geometry.jl:1083-1107).
 __device__ __forceinline__ double inv_beta_gamma(double x, double* d) {
-  if (hi32(x) < 0x3d719799) {  // x < 1e-12: the clamp of beta
+  // x < 1e-12 (the clamp of beta; negative energies) or > 1e100 (x^2 overflows at 1e154)
+  if (uint32_t(hi32(x)) - 0x3d719799u >= 0x54b249adu - 0x3d719799u) {
     const double g = 1.0 + x, b2 = 1.0 - 1.0 / (g * g);
     const double b = ::sqrt(b2 >= 1e-12 ? b2 : 1e-12), r = 1.0 / (b * g);
     *d = b2 >= 1e-12 ? -r / (b2 * g * g * g) - r / g : -r / g;

@@ -129,10 +129,11 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
         }
         __syncwarp();
         ok = ok && (unsigned long long)__double_as_longlong(En) < 0x426d1a94a2000000ull;  // 1e12
-        const double x = (E + En) * half_inv_m, ib = f64::rsqrt(x * (x + 2.0));
+        double dib;
+        const double ib = f64::inv_beta_gamma((E + En) * half_inv_m, &dib);
         dsum = fma(L, ib, dsum);
         // K = dE/dY and half of the segment's decay slope a in its mean energy
-        if (ADJ) work[size_t(s) * 32] = double2{K, L * half_inv_mct * ((x + 1.0) * (ib * ib * ib))};
+        if (ADJ) work[size_t(s) * 32] = double2{K, -(L * half_inv_mct * dib)};
         E = En;
       }
       // the air column from the place on the shared energy grid
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
       __syncwarp();
       const double SN = fma(t, drs, rS[i]), SaN = fma(t, das, aS[i]);
       const double dasF = aS[j + 1] - aS[j], SaF = fma(tj, dasF, aS[j]);
-      const double xa = (E + Ef) * half_inv_m, iba = f64::rsqrt(xa * (xa + 2.0));
+      double diba;
+      const double iba = f64::inv_beta_gamma((E + Ef) * half_inv_m, &diba);
       const double w = f64::div(SN * SaF, S0 * SaN) * f64::exp(-fma(Lair, iba, dsum) * inv_ctau);
       double dlogF = 0.0;
       const double F = gccly_flux(cs, cs129, Ef, active ? P.nq[nd] : 0.0, ADJ ? &dlogF : nullptr);
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
         double nu = 0.0;
         const double cf = coef * f;
         if (coef != 0.0 && f != 0.0 && !edge) {
-          const double hA = Lair * half_inv_mct * ((xa + 1.0) * (iba * iba * iba));
+          const double hA = -(Lair * half_inv_mct * diba);
           const double iE = f64::rcp(E * dle[i]), dSr = drs * iE / SN, dSaN = das * iE / SaN;
           double lam = dSr - dSaN + hA;
           if (!edgeF) {

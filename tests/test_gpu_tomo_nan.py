@@ -52,3 +52,26 @@ def test_nan_node(scene, sign):
     b = dp.TomoModel(phys, grid, (E, q, w0), side_density=2500.0, precision="fp64").vjp(rho, rays, cot)
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("e", [1e300, 1e160, 1e140, np.inf, -np.inf, -1.0, -0.1, -0.05, 0.0, 1e-300])
+def test_node_far_off_the_grid(oracle, e):
+    """Squares of such energies overflow or are negative; the reference's operations give
+    a finite flux.  Against the oracle, whose derivative at an infinite energy is NaN
+    (the node is clamped there and has none)."""
+    import dpgpu as dp
+    orc = oracle.default_physics((oracle.STANDARD_ROCK, oracle.AIR))
+    phys = dp.upload_physics([orc.table(0), orc.table(1)], ["StandardRock", "Air"])
+    grid = dp.VoxelGrid(6, 6, 4, (-30.0, -30.0, 0.0), 10.0)
+    rho = np.random.default_rng(1).uniform(1500.0, 3000.0, grid.ncell)
+    rays = dp.make_rays([[0.0, 0.0, 0.0]] * 5 + [[900.0, 0.0, 0.0]], [0.0, 20.0, 40.0, 60.0, 80.0, 10.0], np.arange(6) * 50.0)
+    nodes = (np.array([0.5, e, 100.0]), np.array([1.0, 0.0, 1.0]), np.array([1.0, 2.0, 3.0]))
+    model = dp.TomoModel(phys, grid, nodes, side_density=2500.0, precision="fp64")
+    flux, grad = model.vjp(rho, rays, np.ones(6))
+    of, og = oracle.tomo_vjp(orc, 0, 1, np.array([6, 6, 4], np.int32), np.array([-30.0, -30.0, 0.0, 10.0, 10.0, 10.0]), rho,
+                             2500.0, rays, nodes, np.ones(6))
+    np.testing.assert_allclose(flux, of, rtol=1e-9, atol=0)
+    if np.isinf(e):
+        assert np.isfinite(grad).all() and (grad != 0).any()
+    else:
+        np.testing.assert_allclose(grad, og, rtol=1e-7, atol=1e-10 * np.abs(og).max())
