@@ -130,7 +130,9 @@ __device__ __forceinline__ void begin(const Tables& tb, const M& m, Walk<N>& k) 
   const Pos p = locate(tb, k.E, k.i);
   const Val v = m.at(p);
   k.i = p.i;
-  k.iE = f64::lt_pos(0.0, k.E) ? f64::rcp(k.E) : 0.0;  // (below the grid no derivative uses it)
+  // (of a normal energy; zero, subnormal and negative ones lie below the grid, where no
+  // derivative uses it)
+  k.iE = f64::hi32(k.E) >= 0x00100000 ? f64::rcp(k.E) : 0.0;
   k.S = v.v;
   k.tau = 0.0;
 #pragma unroll

@@ -41,3 +41,15 @@ def test_sample_of_zero_energy(dp, phys, oracle, orc_phys):  # noqa: F811
     np.testing.assert_allclose(flux, of, rtol=1e-10, atol=0)
     g = _per_cell_first(segs, b.arrays["seg_cell"], jac)
     np.testing.assert_allclose(g, og, rtol=1e-8, atol=1e-12 * np.abs(og).max())
+
+
+@pytest.mark.parametrize("e", [5e-324, 1e-310, 2.2250738585072014e-308, -5e-324, -1.0])
+def test_sample_of_hardly_any_energy(dp, phys, e):  # noqa: F811
+    """Subnormal and negative energies walk as zero does, from below the grid."""
+    out = []
+    for x in (e, 0.0 if e > -1.0 else -1.0 + 2.0 ** -52):
+        b = _batch(dp, phys, [dp.EnergySample(x, 1.0, 1.0), dp.EnergySample(3.0, -1.0, 1.0)], [12.0])
+        out.append(b.run(np.array([0.1, 0.2, 0.0, 0.0, 0.6])))
+    assert np.isfinite(out[0][1]).all() and (out[0][0] > 0).all()
+    for x, y in zip(*out):
+        np.testing.assert_allclose(x, y, rtol=1e-12, atol=0)
