@@ -396,7 +396,8 @@ static __device__ __noinline__ Lane pass1(const Params& P, const Run& R, const T
     const CellMedium c = cell_medium(P, tb, P.seg_cell[j]);
     const double len = P.seg_len[j], E_in = k.E;
     solid_segment(tb, R, c.S, c.rho, c.irho, 0.0, len, k, ratio, tau, g, ok);
-    double v = 0.0, h = 0.0, dv[1] = {0.0}, dh[1] = {0.0};
+    // (a NaN length, which takes no step, leaves the path without a Jacobian)
+    double v = 0.0, h = 0.0, dv[1] = {0.0 * len}, dh[1] = {0.0};
     if (P.corr) vh_cell(P, tb, c, len, E_in, k, v, h, dv, dh);
     S.add(g[0], dv[0], dh[0], k.dE[0]);
     V += v;

@@ -53,3 +53,16 @@ def test_sample_of_hardly_any_energy(dp, phys, e):  # noqa: F811
     assert np.isfinite(out[0][1]).all() and (out[0][0] > 0).all()
     for x, y in zip(*out):
         np.testing.assert_allclose(x, y, rtol=1e-12, atol=0)
+
+
+def test_a_nan_length_spoils_the_jacobian(dp, phys):  # noqa: F811
+    """On resident arrays, where no length is checked: no step, so the path's flux stands,
+    but its whole Jacobian is NaN; the other paths keep theirs."""
+    wf = np.array([0.1, 0.2, 0.0, 0.0, 0.3])
+    good = _batch(dp, phys, _samples(dp, 40, 2), [5.0, 7.0]).to_device().run(wf)
+    b = _batch(dp, phys, _samples(dp, 40, 2), [5.0, np.nan]).to_device()
+    flux, jac = b.run(wf)
+    p = b.arrays["seg_ptr"]
+    np.testing.assert_array_equal(flux, [good[0][0], good[0][1], good[0][0]])
+    np.testing.assert_array_equal(jac[:p[2]], good[1][:p[2]])
+    assert np.isnan(jac[p[2]:p[3]]).all()
