@@ -106,10 +106,11 @@ DP_HD int walk_up(const double* xs, int n, double x, int hint) {
   while (i < n - 2 && !(x < xs[i + 1])) ++i;
   return i;
 }
-// O(1) interval on a uniform log grid, corrected to the bisection answer.
+// O(1) interval on a uniform log grid, corrected to the bisection answer.  (A NaN
+// is converted to the lowest integer: it starts at 0 and ends at the last interval.)
 DP_HD int uniform_interval(const double* lxs, int n, double lx, double lE0, double inv_d) {
   double f = floor((lx - lE0) * inv_d);
-  int i = f < 0.0 ? 0 : (f > double(n - 2) ? n - 2 : int(f));
+  int i = !(f >= 0.0) ? 0 : (f > double(n - 2) ? n - 2 : int(f));
   while (i > 0 && lx < lxs[i]) --i;
   while (i < n - 2 && !(lx < lxs[i + 1])) ++i;
   return i;

@@ -467,7 +467,8 @@ constexpr int kWarps = 4;
 // rays, flux only, 32 nodes: 76 -> 69 us; 8000 rays with the gradient, 70 nodes: 297 ->
 // 285 us.
 __device__ __forceinline__ void node_init(const EvalP& P, int k, const float4* RA, NodeInit* out) {
-  const double E0 = P.nE[k];
+  const bool none = is_nan_bits(P.nE[k]);  // takes no part, as in the FP64 kernel
+  const double E0 = none ? 0.0 : P.nE[k];
   const double *E = P.tab.col(0, DP_COL_E), *LE = P.tab.col(0, DP_COL_LOGE);
   const double *R = P.tab.col(P.rock, DP_COL_CSDA_R), *S = P.tab.col(P.rock, DP_COL_CSDA_S);
   const int last = P.tab.n - 1;
@@ -498,7 +499,7 @@ __device__ __forceinline__ void node_init(const EvalP& P, int k, const float4* R
     i = lo;
   }
   o.i0 = i;
-  o.coef = float(2.0 * P.nw[k] / P.n_nodes);
+  o.coef = none ? 0.0f : float(2.0 * P.nw[k] / P.n_nodes);
   o.q = float(P.nq[k]);
   o.pad = 0.0f;
   out[k] = o;

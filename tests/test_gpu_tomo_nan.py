@@ -75,3 +75,16 @@ def test_node_far_off_the_grid(oracle, e):
         assert np.isfinite(grad).all() and (grad != 0).any()
     else:
         np.testing.assert_allclose(grad, og, rtol=1e-7, atol=1e-10 * np.abs(og).max())
+
+
+@pytest.mark.parametrize("sign", list(NAN))
+def test_nan_node_mixed(scene, sign):
+    dp, phys, grid, rho, rays, cot = scene
+    E = np.geomspace(0.5, 1e5, 40)
+    q, w = np.ones(40), 0.1 * E
+    bad, w0 = E.copy(), w.copy()
+    bad[7], w0[7] = NAN[sign], 0.0
+    a = dp.TomoModel(phys, grid, (bad, q, w), side_density=2500.0, precision="mixed").vjp(rho, rays, cot)
+    b = dp.TomoModel(phys, grid, (E, q, w0), side_density=2500.0, precision="mixed").vjp(rho, rays, cot)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)

@@ -79,3 +79,42 @@ def test_search_ends_at_every_node(tmp_path):
     grids, places, split, wrong = map(int, subprocess.check_output([str(exe)], timeout=120).split())
     assert wrong == 0, (grids, places, wrong)
     assert split > 100, "the grids hold no node whose log the two sides round differently"
+
+
+NAN_SOURCE = r'''
+#include <cmath>
+#include <cstdio>
+#include <limits>
+#include <vector>
+#include "common.cuh"
+int main() {
+  int bad = 0;
+  for (int n : {2, 3, 200}) {
+    std::vector<double> x(n);
+    for (int i = 0; i < n; ++i) x[i] = -7.0 + 0.1 * i;
+    const double nan = std::numeric_limits<double>::quiet_NaN();
+    for (double lx : {nan, -nan, -1e300, 1e300, -std::numeric_limits<double>::infinity(),
+                      std::numeric_limits<double>::infinity()}) {
+      volatile double v = lx;
+      const int i = dp::uniform_interval(x.data(), n, v, x[0], 10.0);
+      if (i < 0 || i > n - 2) ++bad;
+    }
+  }
+  printf("%d\n", bad);
+  return 0;
+}
+'''
+
+
+def test_uniform_search_of_a_nan_stays_on_the_grid(tmp_path):
+    """A double NaN converts to the lowest int (x86 and the device): the search of
+    csrc/common.cuh read the grid from there on."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    if cxx is None or not os.path.exists(os.path.join(include, "cuda_runtime.h")):
+        pytest.skip("needs a host compiler and the CUDA headers")
+    src, exe = tmp_path / "nan.cpp", tmp_path / "nan"
+    src.write_text(NAN_SOURCE)
+    subprocess.check_call([cxx, "-O1", "-std=c++17", "-I", CSRC, "-I", include, str(src), "-o", str(exe)])
+    assert int(subprocess.check_output([str(exe)], timeout=60)) == 0
