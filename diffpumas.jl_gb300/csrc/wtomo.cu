@@ -36,14 +36,16 @@ constexpr double kMaxStep = 60.0;  // CSDA_MAX_STEP_M (src/Tomography.jl:90)
 constexpr int kMaxChunks = 8;      // energy samples per direction <= 32 * kMaxChunks
 constexpr int kThreads = 128;
 
-// Staged column slots: energies, log energies, then per material
-// (rock, water, porous) CSDA and restricted stopping power and straggling,
-// then the air's CSDA stopping power.
-enum Slot { S_E = 0, S_LE, R_CS, R_MS, R_ST, W_CS, W_MS, W_ST, P_CS, P_MS, P_ST, A_CS, kSlots };
+// Column slots: energies, log energies and the CSDA stopping powers of rock,
+// water, porous material and air, which the steps read; then restricted stopping
+// power and straggling of the first three, which a segment's corrections read.
+enum Slot { S_E = 0, S_LE, R_CS, W_CS, P_CS, A_CS, kWalkSlots,
+            R_MS = kWalkSlots, R_ST, W_MS, W_ST, P_MS, P_ST, kSlots };
 
 struct Params {
   TabView tv;                  // FP64 tables in global memory (grid layout)
-  const double* col[kSlots];   // the staged columns (global addresses)
+  const double* col[kSlots];   // the columns (global addresses)
+  int staged;                  // how many of them shared memory holds
   uint32_t col_bytes;
   int porous;                  // porous material present
   double rho_rock, rho_water, rho_porous, porous_top;
@@ -150,11 +152,11 @@ int run(dp_ctx* ctx, const dp_physics* ph, const dp_csda_config* c, const dp_csd
   const int porous = c->porous_material >= 0 ? c->porous_material : c->rock_material;
   const double* cols[wt::kSlots] = {
       v.col(c->rock_material, DP_COL_E),        v.col(c->rock_material, DP_COL_LOGE),
-      v.col(c->rock_material, DP_COL_CSDA_S),   v.col(c->rock_material, DP_COL_MIXED_S),
-      v.col(c->rock_material, DP_COL_STRAG),    v.col(c->water_material, DP_COL_CSDA_S),
+      v.col(c->rock_material, DP_COL_CSDA_S),   v.col(c->water_material, DP_COL_CSDA_S),
+      v.col(porous, DP_COL_CSDA_S),             v.col(c->air_material, DP_COL_CSDA_S),
+      v.col(c->rock_material, DP_COL_MIXED_S),  v.col(c->rock_material, DP_COL_STRAG),
       v.col(c->water_material, DP_COL_MIXED_S), v.col(c->water_material, DP_COL_STRAG),
-      v.col(porous, DP_COL_CSDA_S),             v.col(porous, DP_COL_MIXED_S),
-      v.col(porous, DP_COL_STRAG),              v.col(c->air_material, DP_COL_CSDA_S)};
+      v.col(porous, DP_COL_MIXED_S),            v.col(porous, DP_COL_STRAG)};
   for (int s = 0; s < wt::kSlots; ++s) P.col[s] = cols[s];
   P.col_bytes = uint32_t(v.ld * sizeof(double));
   P.porous = c->porous_material >= 0 ? 1 : 0;
@@ -200,9 +202,14 @@ int run(dp_ctx* ctx, const dp_physics* ph, const dp_csda_config* c, const dp_csd
     return fail(ctx, DP_ERR_ARG, "precision must be DP_PREC_FP64 or DP_PREC_MIXED");
   const bool mixed = precision == DP_PREC_MIXED;
   // the staged FP64 columns with their FP32 copy (mixed), or with the columns
-  // the FP64 walk derives
-  const size_t smem = 16 + (mixed ? size_t(wt::kSlots) * P.col_bytes * 3 / 2
-                                  : size_t(wt64::kCols) * P.col_bytes);
+  // the FP64 walk derives.  Grids of more than 1708 nodes leave no room for all 17
+  // of the latter: the columns that a segment reads once stay in global memory
+  // then, room for 2640 nodes.
+  int optin = 0;
+  DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  auto bytes64 = [&](int staged) { return 16 + size_t(staged + wt64::kDerived) * P.col_bytes; };
+  P.staged = mixed || bytes64(wt::kSlots) <= size_t(optin) ? wt::kSlots : wt::kWalkSlots;
+  const size_t smem = mixed ? 16 + size_t(wt::kSlots) * P.col_bytes * 3 / 2 : bytes64(P.staged);
   const int threads = mixed ? wt::kThreads : wt64::kThreads;
   auto kernel = mixed ? wt32::wtomo_kernel : wt64::wtomo_kernel;
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

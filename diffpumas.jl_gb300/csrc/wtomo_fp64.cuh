@@ -34,7 +34,6 @@ constexpr int kThreads = 32;
 // Columns derived in shared memory: inverse interval widths of log E, and the
 // differences of the CSDA stopping powers over the intervals.
 enum { D_INV = 0, D_R, D_W, D_P, D_A, kDerived };
-constexpr int kCols = wt::kSlots + kDerived;
 
 struct Tables {
   const double* c[wt::kSlots];
@@ -446,15 +445,16 @@ __global__ void __launch_bounds__(kThreads) wtomo_kernel(const __grid_constant__
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
   double* cols = reinterpret_cast<double*>(smem + 16);
-  if (!stage_columns(cols, P.col, wt::kSlots, P.col_bytes, bar, P.wait_iters)) {
+  if (!stage_columns(cols, P.col, P.staged, P.col_bytes, bar, P.wait_iters)) {
     if (threadIdx.x == 0) atomicExch(P.err_flag, 1);
     return;
   }
   const int ld = int(P.col_bytes / 8), n = P.tv.n, lane = threadIdx.x;
   Tables tb;
 #pragma unroll
-  for (int s = 0; s < wt::kSlots; ++s) tb.c[s] = cols + size_t(s) * ld;
-  double* der = cols + size_t(wt::kSlots) * ld;
+  for (int s = 0; s < wt::kSlots; ++s)
+    tb.c[s] = s < wt::kWalkSlots || P.staged == wt::kSlots ? cols + size_t(s) * ld : P.col[s];
+  double* der = cols + size_t(P.staged) * ld;
 #pragma unroll
   for (int s = 0; s < kDerived; ++s) tb.d[s] = der + size_t(s) * ld;
   for (int i = lane; i < n - 1; i += kThreads) {

@@ -25,3 +25,28 @@ def test_mixed_csda(oracle, n):
         assert (np.abs(x - ox) > 2e-6 * np.abs(ox) + atol).mean() <= 2e-3
         np.testing.assert_allclose(x, ox, rtol=1e-3, atol=atol)
         assert x.sum() == pytest.approx(ox.sum(), rel=1e-6)
+
+
+@pytest.mark.parametrize("n", [1709, 2420])
+def test_fp64_water_fraction(oracle, n):
+    """The columns that the corrections read stay out of shared memory from 1709 nodes on."""
+    import test_gpu_wtomo as T
+    dp, orc, phys = _physics(oracle, n)
+    rng = np.random.default_rng(2)
+    wf = rng.uniform(0.0, 0.5, 12)
+    seg = lambda k: [dp.CellSegment(int(c), float(rng.uniform(2.0, 40.0))) for c in rng.integers(1, 13, k)]  # noqa: E731
+    paths = [dp.DirectionalPath(z, 0.0, seg(k), 0.0, 0.0, 5.0 * k, 60.0, True) for k, z in enumerate((0.0, 20.0, 45.0, 65.0))]
+    c = T.CORR["correction"]
+    corr = [1, c["kappa_strag"], c["kappa_hard"], c["resid_a"], c["resid_b"], c["resid_c"], c["resid_d"], 0, 0.0, 0.0]
+    cfg, site = dp.MaterialConfig(1, 3, 2, 1, 2650.0, 1000.0, 1800.0, 20.0), dp.SiteConfig(963.0, 3e4)
+    shallow, samples = np.arange(12) % 2 == 0, T._samples(dp, 33, 4)
+    try:
+        dp.set_csda_correction(**c)
+        f, seg_ptr, cells, jac = dp.csda_flux_batch(phys, shallow, cfg, site, paths, wf, samples)
+    finally:
+        dp.set_csda_correction(enabled=False)
+    of, og = T._oracle(oracle, orc, wf, paths, samples, corr, shallow.astype(np.uint8), [0, 2, 1, 0],
+                       (2650.0, 1000.0, 1800.0, 20.0))
+    assert (of > 0).all()
+    np.testing.assert_allclose(f, of, rtol=1e-10, atol=0)
+    np.testing.assert_allclose(T._per_cell_first(seg_ptr, cells, jac), og, rtol=1e-8, atol=1e-12 * np.abs(og).max())
