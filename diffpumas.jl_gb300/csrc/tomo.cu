@@ -428,6 +428,7 @@ struct EvalP {
   const float4* geom;
   const double2* star;  // per ray: cos_theta_star and its 1.29 power
   double2* work;        // FP64 adjoint: per resident warp, segment and lane
+  int staged;           // FP64: table columns in shared memory
   const NodeInit* node0;
   const int32_t* order;
   int ld32;
@@ -1102,9 +1103,15 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
     DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
     const size_t most = size_t(optin) - 64;  // the kernel's own barrier
-    while (warps > 1 && eval64_smem(P.tab.ld, P.seg_cap, warps, adj) > most) warps /= 2;
-    smem = eval64_smem(P.tab.ld, P.seg_cap, warps, adj);
-    if (smem > most) return fail(ctx, DP_ERR_ARG, "ray too long for the FP64 kernel");
+    // A warp per SM partition comes before the columns that a ray reads at its ends
+    // only: those stay in global memory on grids of some thousand nodes.
+    auto fits = [&](int staged) {
+      P.staged = staged;
+      smem = eval64_smem(staged, P.tab.ld, P.seg_cap, warps, adj);
+      return smem <= most;
+    };
+    while (!fits(T_NCOL) && !fits(T_SEGCOL) && warps > 1) warps /= 2;
+    if (smem > most) return fail(ctx, DP_ERR_ARG, "energy grid too large or ray too long for the FP64 kernel");
     auto kernel = adj ? eval64_kernel<true> : eval64_kernel<false>;
     DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));

@@ -20,12 +20,13 @@
 // about 450.  4096 rays of the 64x64x32 grid, 32 nodes, flux and J^T r: kernel
 // 6.94 -> 0.75 ms.
 
-// Shared memory: six staged columns, two derived ones, then per warp the
-// lengths and grammages of the ray's segments and (ADJ) the 32 x 33 tile.
-enum { T_E = 0, T_LOGE, T_RS, T_RR, T_AS, T_AR, T_NCOL, T_RINV = T_NCOL, T_DLE, T_ALL };
+// Shared memory: the staged columns (all six, or the three that the segments read,
+// the others then in global memory), two derived ones, then per warp the lengths and
+// grammages of the ray's segments and (ADJ) the 32 x 33 tile.
+enum { T_E = 0, T_LOGE, T_RR, T_SEGCOL, T_RS = T_SEGCOL, T_AS, T_AR, T_NCOL };
 constexpr int kTile = 32 * 33;
-__host__ __device__ inline size_t eval64_smem(int ld, int seg_cap, int warps, bool adj) {
-  return (size_t(T_ALL) * ld + size_t(warps) * (2 * size_t(seg_cap) + (adj ? kTile : 0))) * sizeof(double);
+inline size_t eval64_smem(int staged, int ld, int seg_cap, int warps, bool adj) {
+  return (size_t(staged + 2) * ld + size_t(warps) * (2 * size_t(seg_cap) + (adj ? kTile : 0))) * sizeof(double);
 }
 __device__ __forceinline__ bool is_nan_bits(double x) {
   return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
@@ -37,23 +38,24 @@ __global__ void __launch_bounds__(kWarps * 32) eval64_kernel(EvalP P) {
   __shared__ uint64_t mbar;
   const int ld = P.tab.ld, n = P.tab.n;
   const double* src[T_NCOL] = {P.tab.col(0, DP_COL_E),          P.tab.col(0, DP_COL_LOGE),
-                               P.tab.col(P.rock, DP_COL_CSDA_S), P.tab.col(P.rock, DP_COL_CSDA_R),
+                               P.tab.col(P.rock, DP_COL_CSDA_R), P.tab.col(P.rock, DP_COL_CSDA_S),
                                P.tab.col(P.air, DP_COL_CSDA_S),  P.tab.col(P.air, DP_COL_CSDA_R)};
-  if (!stage_columns(smem, src, T_NCOL, uint32_t(ld * sizeof(double)), &mbar, P.wait_iters)) {
+  if (!stage_columns(smem, src, P.staged, uint32_t(ld * sizeof(double)), &mbar, P.wait_iters)) {
     if (threadIdx.x == 0) atomicExch(P.err_flag, 1);
     return;
   }
-  const double *tE = smem + T_E * ld, *tlE = smem + T_LOGE * ld;
-  const double *rS = smem + T_RS * ld, *rR = smem + T_RR * ld;
-  const double *aS = smem + T_AS * ld, *aR = smem + T_AR * ld;
-  double *rinv = smem + T_RINV * ld, *dle = smem + T_DLE * ld;
+  const bool all = P.staged == T_NCOL;
+  const double *tE = smem + T_E * ld, *tlE = smem + T_LOGE * ld, *rR = smem + T_RR * ld;
+  const double* rS = all ? smem + T_RS * ld : src[T_RS];
+  const double *aS = all ? smem + T_AS * ld : src[T_AS], *aR = all ? smem + T_AR * ld : src[T_AR];
+  double *rinv = smem + P.staged * ld, *dle = rinv + ld;
   for (int i = threadIdx.x; i < n - 1; i += blockDim.x) {
     rinv[i] = 1.0 / (rR[i + 1] - rR[i]);
     dle[i] = tlE[i + 1] - tlE[i];
   }
   __syncthreads();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = P.seg_cap;
-  double* sL = smem + size_t(T_ALL) * ld + size_t(warp) * (2 * size_t(cap) + (ADJ ? kTile : 0));
+  double* sL = dle + ld + size_t(warp) * (2 * size_t(cap) + (ADJ ? kTile : 0));
   double* sG = sL + cap;    // grammage rho L
   double* tile = sG + cap;  // [segment & 31][lane]
   double2* work = ADJ ? P.work + (size_t(blockIdx.x) * warps + warp) * size_t(cap) * 32 + lane : nullptr;

@@ -50,3 +50,27 @@ def test_fp64_water_fraction(oracle, n):
     assert (of > 0).all()
     np.testing.assert_allclose(f, of, rtol=1e-10, atol=0)
     np.testing.assert_allclose(T._per_cell_first(seg_ptr, cells, jac), og, rtol=1e-8, atol=1e-12 * np.abs(og).max())
+
+
+@pytest.mark.parametrize("n", [3400, 5000])
+def test_fp64_tomography(oracle, n):
+    """The columns that a ray reads at its ends stay out of shared memory (3400 nodes:
+    with the gradient only), and two warps find room where four do otherwise (5000)."""
+    import dpgpu as dp
+    orc = oracle.default_physics((oracle.STANDARD_ROCK, oracle.AIR), n=n)
+    phys = dp.upload_physics([orc.table(0), orc.table(1)], ["StandardRock", "Air"])
+    grid = dp.VoxelGrid(40, 36, 20, (-200.0, -180.0, 0.0), 10.0)
+    rng = np.random.default_rng(4)
+    rho = rng.uniform(800.0, 3200.0, grid.ncell)
+    o = np.column_stack([rng.uniform(-190, 190, 12), rng.uniform(-170, 170, 12), np.zeros(12)])
+    rays = dp.make_rays(o, rng.uniform(0.0, 85.0, 12), rng.uniform(0.0, 360.0, 12))
+    E = np.concatenate([[2e-4, 1e-3, 9e8, 2e9], np.geomspace(1e-2, 1e8, 37)])
+    nodes = (E, np.where(np.arange(len(E)) % 3, 0.0, 1.0), 0.1 * E)
+    cot = rng.uniform(0.5, 1.5, len(rays))
+    model = dp.TomoModel(phys, grid, nodes, side_density=2500.0, precision="fp64")
+    flux, grad = model.vjp(rho, rays, cot)
+    dims, geom = np.array([grid.nx, grid.ny, grid.nz], np.int32), np.array([*grid.origin, *grid.pitch])
+    of, og = oracle.tomo_vjp(orc, 0, 1, dims, geom, rho, 2500.0, rays, nodes, cot)
+    np.testing.assert_allclose(flux, of, rtol=1e-9, atol=0)
+    np.testing.assert_array_equal(model.forward(rho, rays), flux)
+    np.testing.assert_allclose(grad, og, rtol=1e-7, atol=1e-10 * np.abs(og).max())
