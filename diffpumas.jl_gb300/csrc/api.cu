@@ -25,10 +25,17 @@ void* scratch(dp_ctx* ctx, size_t bytes, int slot) {
   }
   p = nullptr;
   have = 0;
-  size_t want = bytes + bytes / 4 + 256;
-  if (cudaMalloc(&p, want) != cudaSuccess) return nullptr;
-  have = want;
-  return p;
+  const size_t most = ctx->dbg_scratch < 0 ? SIZE_MAX : size_t(ctx->dbg_scratch);
+  // with room to grow, where the device has it
+  for (size_t want : {bytes + bytes / 4 + 256, bytes + 256}) {
+    if (want <= most && cudaMalloc(&p, want) == cudaSuccess) {
+      have = want;
+      return p;
+    }
+    cudaGetLastError();  // the caller may go on with less
+    p = nullptr;
+  }
+  return nullptr;
 }
 static cudaEvent_t take_event(dp_ctx* ctx) {
   cudaEvent_t e = nullptr;
@@ -181,6 +188,12 @@ int dp_set_debug_limits(dp_ctx* c, int step_cap, int event_cap, int wait_iters) 
   c->dbg_step_cap = step_cap < 0 ? -1 : step_cap;
   c->dbg_event_cap = event_cap < 0 ? -1 : event_cap;
   c->dbg_wait = wait_iters < 0 ? -1 : wait_iters;
+  return DP_OK;
+}
+
+int dp_set_debug_scratch(dp_ctx* c, long long max_bytes) {
+  if (!c) return DP_ERR_ARG;
+  c->dbg_scratch = max_bytes;
   return DP_OK;
 }
 

@@ -58,6 +58,7 @@ struct dp_ctx {
   // the default (2,000,000 transport steps, 100,000 hard events per mixed
   // step, dp::kStageWait polls of a table-staging wait).
   int dbg_step_cap = -1, dbg_event_cap = -1, dbg_wait = -1;
+  long long dbg_scratch = -1;  // bytes of a scratch slot (dp_set_debug_scratch)
 };
 
 namespace dp {

@@ -1116,12 +1116,16 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
     DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
     blocks = std::min<long>((pa->n_rays + warps - 1) / warps, long(std::max(per_sm, 1)) * n_sm);
-    if (adj) work = size_t(blocks) * warps * P.seg_cap * 32 * sizeof(double2);
   }
-  // slot 1: node starts, then the Jacobian values and the FP64 adjoint's terms
-  size_t need = size_t(P.n_nodes) * sizeof(NodeInit) + size_t(pa->nnz + 1) * 8 + work + 2048;
+  // slot 1: the Jacobian values and the FP64 adjoint's terms, 512 bytes per segment
+  // slot of each warp in flight (0.2 GB for 250 slots): fewer CTAs where the device
+  // has no room for them
   Arena A;
-  A.base = static_cast<char*>(scratch(ctx, need, 1));
+  for (;; blocks = (blocks + 1) / 2) {
+    if (precision == 0 && adj) work = size_t(blocks) * warps * P.seg_cap * 32 * sizeof(double2);
+    A.base = static_cast<char*>(scratch(ctx, size_t(pa->nnz + 1) * 8 + work + 2048, 1));
+    if (A.base || work == 0 || blocks == 1) break;
+  }
   A.cap = ctx->slot_bytes[1];
   if (!A.base) return fail(ctx, DP_ERR_ALLOC, "scratch allocation failed");
   void* jbuf = nullptr;

@@ -176,6 +176,7 @@ PROTOTYPES = {
     "dp_set_blocking": (_I, [_P, _I]),
     "dp_sync": (_I, [_P]),
     "dp_set_debug_limits": (_I, [_P, _I, _I, _I]),
+    "dp_set_debug_scratch": (_I, [_P, C.c_longlong]),
     "dp_mc_thread_choices": (_I, [_I, _VP, _I]),
     "dp_set_mc_threads": (_I, [_P, _I, _I, _I]),
     "dp_get_mc_threads": (_I, [_P, _I, _I, C.POINTER(_I)]),

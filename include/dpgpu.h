@@ -106,6 +106,10 @@ int dp_sync(dp_ctx* ctx);
  * leaves).  A negative value restores the default.  Every limit ends its loop
  * with a status the call reports (DP_ERR_STATE); none of them faults. */
 int dp_set_debug_limits(dp_ctx* ctx, int step_cap, int event_cap, int wait_iters);
+/* The largest scratch slot (bytes) that this context may allocate from here on, for tests of
+ * calls that run short of device memory; negative: no limit.  A call that cannot
+ * do with it reports DP_ERR_ALLOC. */
+int dp_set_debug_scratch(dp_ctx* ctx, long long max_bytes);
 
 /* ------------------------------------------------------------------ launch shapes
  * CTA size of the persistent transport kernels per kernel family and
@@ -689,7 +693,10 @@ int dp_tomo_paths_csr(const dp_paths* paths, int64_t* row_ptr, int32_t* col, dou
 #define DP_PREC_MIXED 1  /* per-segment work in FP32, FP64 range carry and flux integral */
 /* One evaluation on device pointers (node arrays of tp are device pointers):
  * flux[n_rays]; if cot/grad are given, grad[ncell] = J^T cot (deterministic);
- * if jac is given, the Jacobian values in the CSR order of the paths. */
+ * if jac is given, the Jacobian values in the CSR order of the paths.
+ * Scratch of a gradient: 8 bytes per segment, and in FP64 512 bytes per slot of the
+ * longest segment list and ray in flight (0.2 GB for 250 slots; less, and slower,
+ * where the device has no room).  It stays with the context. */
 int dp_tomo_eval_dev(dp_ctx* ctx, const dp_physics* phys, const dp_paths* paths,
                      const dp_tomo_params* tp, const double* rho, const double* cot,
                      double* flux, double* grad_rho, double* jac, int precision);
