@@ -429,7 +429,7 @@ struct EvalP {
   const double2* star;  // per ray: cos_theta_star and its 1.29 power
   double2* work;        // FP64 adjoint: per resident warp, segment and lane
   int staged;           // FP64: table columns in shared memory
-  const NodeInit* node0;
+  const NodeInit* node0;  // mixed: the node starts, null where each block computes them
   const int32_t* order;
   int ld32;
   int rock, air, n_nodes, seg_cap;
@@ -582,8 +582,12 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
   float* sG = fsm + size_t(2 * kNC32) * ld + size_t(warp) * cap * 3;  // grammage rho L
   float* sL = sG + cap;                                              // length L
   float* sJ = sL + cap;                                              // Jacobian accumulator
-  NodeInit* snode = reinterpret_cast<NodeInit*>(fsm + size_t(2 * kNC32) * ld + size_t(kWarps) * cap * 3);
-  for (int k = threadIdx.x; k < P.n_nodes; k += blockDim.x) node_init(P, k, RA, snode);
+  const NodeInit* snode = P.node0;
+  if (!snode) {
+    NodeInit* own = reinterpret_cast<NodeInit*>(fsm + size_t(2 * kNC32) * ld + size_t(kWarps) * cap * 3);
+    for (int k = threadIdx.x; k < P.n_nodes; k += blockDim.x) node_init(P, k, RA, own);
+    snode = own;
+  }
   __syncthreads();
   const float inv_m = float(1.0 / P.mass), inv_ctau = float(1.0 / P.ctau);
   const float Lair_c = float(P.H - P.zmax), Gair_c = float(1.205 * 12e3 * P.air_dexp);
@@ -733,6 +737,13 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
       for (int s = lane; s < nseg; s += 32) P.jval32[off + s] = sJ[s];
     __syncwarp();
   }
+}
+
+// The node starts of quadratures that the blocks of eval32_kernel have no room for.
+__global__ void node_start_kernel(EvalP P, NodeInit* out) {
+  const float4* RA = reinterpret_cast<const float4*>(P.tab32 + (size_t(P.rock) * kNC32Rows + kNC32) * P.ld32);
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n_nodes; k += gridDim.x * blockDim.x)
+    node_init(P, k, RA, out);
 }
 
 // J^T r over the precomputed CSC permutation, every bucket in a fixed order
@@ -1117,13 +1128,22 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
     blocks = std::min<long>((pa->n_rays + warps - 1) / warps, long(std::max(per_sm, 1)) * n_sm);
   }
+  size_t starts = 0;
+  if (precision) {
+    // the node starts beside the segment lists where they fit (some 6700 nodes)
+    const size_t lists = size_t(2 * kNC32) * P.ld32 * 4 + size_t(kWarps) * P.seg_cap * 3 * 4;
+    const size_t nodes = size_t(P.n_nodes) * sizeof(NodeInit), most = 220 * 1024;
+    if (lists > most) return fail(ctx, DP_ERR_ARG, "energy grid too large or ray too long for the mixed kernel");
+    if (lists + nodes > most) starts = nodes;
+    smem = starts ? lists : lists + nodes;
+  }
   // slot 1: the Jacobian values and the FP64 adjoint's terms, 512 bytes per segment
   // slot of each warp in flight (0.2 GB for 250 slots): fewer CTAs where the device
   // has no room for them
   Arena A;
   for (;; blocks = (blocks + 1) / 2) {
     if (precision == 0 && adj) work = size_t(blocks) * warps * P.seg_cap * 32 * sizeof(double2);
-    A.base = static_cast<char*>(scratch(ctx, size_t(pa->nnz + 1) * 8 + work + 2048, 1));
+    A.base = static_cast<char*>(scratch(ctx, size_t(pa->nnz + 1) * 8 + work + starts + 2048, 1));
     if (A.base || work == 0 || blocks == 1) break;
   }
   A.cap = ctx->slot_bytes[1];
@@ -1152,10 +1172,14 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
       eval64_kernel<false><<<int(blocks), warps * 32, smem, ctx->stream>>>(P);
     }
   } else {
-    smem = size_t(2 * kNC32) * P.ld32 * 4 + size_t(kWarps) * P.seg_cap * 3 * 4 +
-           size_t(P.n_nodes) * sizeof(NodeInit);
-    if (smem > 220 * 1024) return fail(ctx, DP_ERR_ARG, "ray too long for the mixed kernel");
     P.jval32 = static_cast<float*>(jbuf);
+    if (starts) {
+      NodeInit* out = A.take<NodeInit>(P.n_nodes);
+      if (!out) return fail(ctx, DP_ERR_ALLOC, "scratch allocation failed");
+      node_start_kernel<<<(P.n_nodes + 127) / 128, 128, 0, ctx->stream>>>(P, out);
+      ++ctx->launches;
+      P.node0 = out;
+    }
     if (adj) eval32_kernel<true><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
     else eval32_kernel<false><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
   }
@@ -1595,7 +1619,8 @@ extern "C" int dp_tomo_eval_noalloc_dev(dp_ctx* ctx, const dp_physics* ph, const
   P.jval32 = jac;  // every segment's value is written before the gather reads it
   const size_t smem = size_t(2 * kNC32) * P.ld32 * 4 + size_t(kWarps) * P.seg_cap * 3 * 4 +
                       size_t(P.n_nodes) * sizeof(NodeInit);
-  if (smem > 220 * 1024) return fail(ctx, DP_ERR_ARG, "ray too long for the mixed kernel");
+  if (smem > 220 * 1024)
+    return fail(ctx, DP_ERR_ARG, "energy grid too large, ray too long or too many nodes for the allocation-free form");
   const long blocks = std::min<long>((pa->n_rays + kWarps - 1) / kWarps, 152L * 16);
   const bool adj = cot != nullptr;
   if (adj) {

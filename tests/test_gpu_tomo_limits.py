@@ -43,3 +43,21 @@ def test_fp64_gradient_short_of_scratch():
     dp.check(dp.load().dp_set_debug_scratch(other.h, -1), other.h)
     for a, b in zip(paths.eval(rho, cot, precision="fp64")[:2], full):
         np.testing.assert_array_equal(a.cpu().numpy(), b)
+
+
+def test_mixed_with_thousands_of_nodes():
+    """90 copies of 100 nodes have the 100 nodes' mean.  A node's coefficient 2 w / N is
+    rounded to FP32 on either side (2^-23 together, 2^-22 allowed), and a segment's
+    entry is summed in FP32 over 282 groups of nodes of one sign (282 2^-24)."""
+    import dpgpu as dp
+    E, q = np.geomspace(1.0, 1e5, 100), np.where(np.arange(100) % 2, 1.0, -1.0)
+    out = []
+    for k in (1, 90):
+        paths, rho, cot = _paths(dp, dp.default_context(), [np.tile(x, k) for x in (E, q, 0.1 * E)], 60)
+        f, g, _ = paths.eval(rho, cot, precision="mixed")
+        np.testing.assert_array_equal(paths.eval(rho, precision="mixed")[0].cpu().numpy(), f.cpu().numpy())
+        out.append((f.cpu().numpy(), g.cpu().numpy()))
+    (f0, g0), (f1, g1) = out
+    assert (f0 > 0).all()
+    np.testing.assert_allclose(f1, f0, rtol=2.0 ** -22, atol=0)
+    np.testing.assert_allclose(g1, g0, rtol=0, atol=282 * 2.0 ** -24 * np.abs(g0).max())
