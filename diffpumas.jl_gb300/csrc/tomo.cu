@@ -429,7 +429,7 @@ struct EvalP {
   const double2* star;  // per ray: cos_theta_star and its 1.29 power
   double2* work;        // FP64 adjoint: per resident warp, segment and lane
   int staged;           // FP64: table columns in shared memory
-  const NodeInit* node0;  // mixed: the node starts, null where each block computes them
+  const NodeInit* node0;  // mixed: the node starts where the blocks have no room for them
   const int32_t* order;
   int ld32;
   int rock, air, n_nodes, seg_cap;
@@ -554,7 +554,9 @@ __device__ __forceinline__ float4 walk_rows(const float4* RA, int n, float yh, i
   return r;
 }
 
-template <bool ADJ>
+// STARTS: the node starts are in P.node0 (a kernel of its own: 0.9 % of a Gauss-Newton
+// inversion where a pointer chose).
+template <bool ADJ, bool STARTS = false>
 __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
   extern __shared__ __align__(16) float fsm[];
   __shared__ uint64_t mbar;
@@ -582,12 +584,10 @@ __global__ void __launch_bounds__(kWarps * 32, 8) eval32_kernel(EvalP P) {
   float* sG = fsm + size_t(2 * kNC32) * ld + size_t(warp) * cap * 3;  // grammage rho L
   float* sL = sG + cap;                                              // length L
   float* sJ = sL + cap;                                              // Jacobian accumulator
-  const NodeInit* snode = P.node0;
-  if (!snode) {
-    NodeInit* own = reinterpret_cast<NodeInit*>(fsm + size_t(2 * kNC32) * ld + size_t(kWarps) * cap * 3);
+  NodeInit* own = reinterpret_cast<NodeInit*>(fsm + size_t(2 * kNC32) * ld + size_t(kWarps) * cap * 3);
+  if (!STARTS)
     for (int k = threadIdx.x; k < P.n_nodes; k += blockDim.x) node_init(P, k, RA, own);
-    snode = own;
-  }
+  const NodeInit* snode = STARTS ? P.node0 : own;
   __syncthreads();
   const float inv_m = float(1.0 / P.mass), inv_ctau = float(1.0 / P.ctau);
   const float Lair_c = float(P.H - P.zmax), Gair_c = float(1.205 * 12e3 * P.air_dexp);
@@ -1179,9 +1179,14 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
       node_start_kernel<<<(P.n_nodes + 127) / 128, 128, 0, ctx->stream>>>(P, out);
       ++ctx->launches;
       P.node0 = out;
+      auto kernel = adj ? eval32_kernel<true, true> : eval32_kernel<false, true>;
+      DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      kernel<<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
+    } else if (adj) {
+      eval32_kernel<true><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
+    } else {
+      eval32_kernel<false><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
     }
-    if (adj) eval32_kernel<true><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
-    else eval32_kernel<false><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
   }
   DP_CHECK_CUDA(ctx, cudaGetLastError());
   timed_end(ctx, adj ? "tomo_adjoint" : "tomo_forward");
