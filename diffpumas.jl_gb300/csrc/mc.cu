@@ -219,20 +219,19 @@ Layout make_layout(const dp_mixture* const* media, int n_media, size_t esize) {
   }
   L.ld = pad_elems(L.n, esize);
   L.ldk = pad_elems(L.nk, esize);
-  // elements, then the index-table origins and widths (2 doubles per column),
-  // then (FP64) the elements' DCS constants
+  // elements, then the index-table origins and widths (FP32: 2 doubles per column)
+  // or the elements' DCS constants (FP64)
   int nel = 0;
   for (int k = 0; k < n_media; ++k) nel = std::max(nel, media[k]->nel);
-  L.o_phys = uint32_t((kEldOffset + (esize == 8 ? nel * kEldStride : 0)) * sizeof(double));
+  L.o_phys = uint32_t((kMaxEl * kElStride + (esize == 8 ? nel * kEldStride : 2 * I_NCOL)) * sizeof(double));
   // FP64 media carry the inverse interval widths too (pack_derived)
   const int dp = esize == 8 ? X_NCOL : 0, dk = esize == 8 ? 1 : 0;
   L.o_ker = L.o_phys + uint32_t(size_t(MC_LB1 + 2 * L.slots + dp) * L.ld * esize);
   L.o_idx = L.o_ker + uint32_t(size_t(K_NCOL + dk) * L.ldk * esize);
-  L.nbp = kIdxBinsPhys;
-  L.nbk = kIdxBinsKer;
-  uint32_t idx_bytes = uint32_t((2 * kIdxBinsPhys + 2 * kIdxBinsKer) * sizeof(int16_t));
+  // (the FP64 inverse lookups walk from the step's own interval)
+  uint32_t idx_bytes = esize == 8 ? 0 : uint32_t((2 * kIdxBinsPhys + 2 * kIdxBinsKer) * sizeof(int16_t));
   L.o_elf = L.o_idx + (idx_bytes + 15) / 16 * 16;
-  L.med_bytes = L.o_elf + uint32_t(kMaxEl * kElfStride * sizeof(float));
+  L.med_bytes = L.o_elf + (esize == 8 ? 0 : uint32_t(kMaxEl * kElfStride * sizeof(float)));
   const dp_physics* ph = a->phys;
   L.uniform = ph->view.uniform;
   L.lE0 = ph->view.lE0;
@@ -300,6 +299,11 @@ static void pack(const dp_mixture* m, const Layout& L, unsigned char* out) {
   }
   R* K = reinterpret_cast<R*>(out + L.o_ker);
   for (int c = 0; c < K_NCOL; ++c) put(K + size_t(c) * L.ldk, m->kcols.data() + size_t(c) * m->nk, m->nk);
+  if constexpr (sizeof(R) == 8) {
+    pack_dcs(m, reinterpret_cast<double*>(out) + kMaxEl * kElStride);
+    pack_derived(m, L, P, K);
+    return;
+  }
   // FP32 element table of the cooperative DCS sums
   float* elf = reinterpret_cast<float*>(out + L.o_elf);
   for (int e = 0; e < m->nel; ++e) {
@@ -311,10 +315,6 @@ static void pack(const dp_mixture* m, const Layout& L, unsigned char* out) {
     f[3] = float(x[3]);
     f[4] = float(kAvogadro / (x[1] * 0.001));
     f[5] = float(x[4]);  // nuclear RMS radius (DEL polar angles)
-  }
-  if constexpr (sizeof(R) == 8) {
-    pack_dcs(m, reinterpret_cast<double*>(out) + kEldOffset);
-    pack_derived(m, L, P, K);
   }
   // index tables of the inverse lookups (origins and widths in R)
   R* prm = reinterpret_cast<R*>(reinterpret_cast<double*>(out) + kMaxEl * kElStride);

@@ -61,8 +61,7 @@ struct Layout {
   double lE0, inv_dlE;
   int kuniform;        // MIXED kernel energies: the uniform log grid refined 8-fold
   double kinv_dlE;     // 1 / log step of the kernel energies
-  uint32_t o_idx;      // byte offset of the inverse-lookup index tables (int16)
-  int nbp, nbk;        // index bins of the physics and kernel columns
+  uint32_t o_idx;      // byte offset of the inverse-lookup index tables (int16; FP32 media)
   uint32_t o_elf;      // byte offset of the FP32 element table (kElfStride floats each)
 };
 // FP32 element table for the cooperative DCS sums and the FP32 polar angles:
@@ -70,8 +69,8 @@ struct Layout {
 constexpr int kElfStride = 8;
 
 // FP64 media: per-element constants of the warp-wide FP64 DCS sums (filled by
-// pack_medium): everything in the cross sections that depends on the element
-// and the muon mass only.  They follow the index origins, kEldStride doubles
+// pack_dcs): everything in the cross sections that depends on the element
+// and the muon mass only.  They follow the elements, kEldStride doubles
 // per element.
 enum EldCol {
   EL_Z = 0, EL_A, EL_I, EL_SCALE,  // EL_SCALE: mass fraction x N_A / (A 1e-3)
@@ -96,8 +95,6 @@ enum EldCol {
 // origin and inverse width (two doubles) follow the elements.
 enum IdxCol { I_CR = 0, I_MR, I_KR, I_KH, I_NCOL };
 constexpr int kIdxBinsPhys = 256, kIdxBinsKer = 1024;
-// Doubles from an FP64 medium's elements to its DCS constants.
-constexpr int kEldOffset = kMaxEl * kElStride + 2 * I_NCOL;
 struct MedInfo {
   int nm, nel;
   double frac[kMaxMix];
@@ -455,11 +452,14 @@ __device__ __forceinline__ KLoc<R> klocate_idx(const Med<R>& m, int xcol, R x, i
   L.f = d == R(0) ? R(0) : (x - xs[i]) / d;
   return L;
 }
+// A kernel column at an energy, and at a range or hazard.
 template <class R>
-__device__ __forceinline__ R klookup(const Med<R>& m, int xcol, int ycol, R x, int* status) {
-  if (xcol == K_E) return kat(m.kcol(ycol), m.nk, klocate_e(m, x, status));
-  if (xcol == K_R || xcol == K_H) return kat(m.kcol(ycol), m.nk, klocate_idx(m, xcol, x, status));
-  return kat(m.kcol(ycol), m.nk, klocate(m.kcol(xcol), m.nk, x, status));
+__device__ __forceinline__ R klookup_e(const Med<R>& m, int ycol, R x, int* status) {
+  return kat(m.kcol(ycol), m.nk, klocate_e(m, x, status));
+}
+template <class R>
+__device__ __forceinline__ R klookup_idx(const Med<R>& m, int xcol, int ycol, R x, int* status) {
+  return kat(m.kcol(ycol), m.nk, klocate_idx(m, xcol, x, status));
 }
 
 // Terms of one hard-event DCS sum spread over a warp: per element one
@@ -829,7 +829,7 @@ static __device__ __noinline__ bool del_begin(const Med<R>& m, const Consts& C, 
                                               int* status, DelOut* out, double* anc_out,
                                               double* denom) {
   *out = DelOut{k, 1.0, 0, -1};
-  double sigma = double(klookup(m, K_E, K_SIG, R(k), status));
+  double sigma = double(klookup_e(m, K_SIG, R(k), status));
   if (!(sigma > 0.0)) {
     *status |= ST_ZERO_RATE;
     return false;
@@ -862,7 +862,7 @@ static __device__ __noinline__ bool del_begin32(const Med<float>& m, const Const
                                                 int* status, DelOutT<float>* out, float* anc_out,
                                                 float* q_out, float* denom) {
   *out = DelOutT<float>{k, 1.f, 0, -1};
-  const float sigma = klookup(m, K_E, K_SIG, k, status);
+  const float sigma = klookup_e(m, K_SIG, k, status);
   if (!(sigma > 0.f)) {
     *status |= ST_ZERO_RATE;
     return false;
@@ -1010,12 +1010,12 @@ __device__ __forceinline__ bool mixed_run_in(const Med<R>& m, const Consts& C, S
     }
     KLoc<R> Lk = klocate_e(m, k, &s.status);
     R ri = kat(m.kcol(K_R), nk, Lk), hi = kat(m.kcol(K_H), nk, Lk);
-    R rtc = fmax(R(0), klookup(m, K_E, K_R, x.r2, &s.status) - ri);
+    R rtc = fmax(R(0), klookup_e(m, K_R, x.r2, &s.status) - ri);
     R eg = fmin(x.a, rtc);
-    R endpoint = eg == rtc ? x.r2 : fmax(k, klookup(m, K_R, K_E, ri + eg, &s.status));
+    R endpoint = eg == rtc ? x.r2 : fmax(k, klookup_idx(m, K_R, K_E, ri + eg, &s.status));
     R eventh = hi + expo<R>(g);
-    bool occurs = eventh < klookup(m, K_E, K_H, endpoint, &s.status);
-    R pre = occurs ? fmax(k, klookup(m, K_H, K_E, eventh, &s.status)) : endpoint;
+    bool occurs = eventh < klookup_e(m, K_H, endpoint, &s.status);
+    R pre = occurs ? fmax(k, klookup_idx(m, K_H, K_E, eventh, &s.status)) : endpoint;
     KLoc<R> Lp = klocate_e(m, pre, &s.status);
     R dx = occurs ? fmax(R(0), kat(m.kcol(K_R), nk, Lp) - ri) : eg;
     R dt;
@@ -1499,13 +1499,13 @@ __device__ bool straggled_step(const Med<R>& m, const Consts& C, State<R>& s, co
   }
   bool del = false, ehs = false;
   R X_del = R(CUDART_INF), k_del = R(0), X_ehs = R(CUDART_INF), k_ehs = R(0);
-  R rate = fmax(klookup(m, K_E, K_SIG, ki, &s.status), klookup(m, K_E, K_SIG, kf, &s.status));
+  R rate = fmax(klookup_e(m, K_SIG, ki, &s.status), klookup_e(m, K_SIG, kf, &s.status));
   if (rate > R(0)) {
     R cand = expo<R>(g) / rate;
     if (cand < dX) {
       R kh = inv_range(m, MC_MR, Xi + cand);
       R pre = ki + ratio * fabs(kh - ki);
-      if (pre > R(0) && uni<R>(g) <= klookup(m, K_E, K_SIG, pre, &s.status) / rate) {
+      if (pre > R(0) && uni<R>(g) <= klookup_e(m, K_SIG, pre, &s.status) / rate) {
         del = true;
         X_del = cand;
         k_del = pre;

@@ -129,9 +129,6 @@ __device__ __forceinline__ KLoc<double> klocate_from(const Med<double>& m, int x
   L.f = d == 0.0 ? 0.0 : f64::div(x - xs[i], d);
   return L;
 }
-__device__ __forceinline__ double klookup(const Med<double>& m, int xcol_, int ycol, double x, int* status) {
-  return kat(m.kcol(ycol), m.nk, klocate_e(m, x, status));  // the callers' axis is the energy
-}
 // Hazard rate per grammage at an energy.
 __device__ __forceinline__ double rate_at(const Med<double>& m, double x, double lx, int* status) {
   return kat(m.kcol(K_SIG), m.nk, klocate_log(m, x, lx, status));

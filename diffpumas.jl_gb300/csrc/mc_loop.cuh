@@ -427,7 +427,7 @@ __device__ __forceinline__ void transport_histories(G& geo, const Consts& C,
         const Med<R>& m = geo.medium(__shfl_sync(0xffffffffu, h.x.medium, from));
         const double anc = __shfl_sync(0xffffffffu, h.x.anc, from);
         const double q = __shfl_sync(0xffffffffu, h.x.q, from);
-        const double total = del64_sum(m.el + kEldOffset, m.nel, C.mass, anc, q, buf);
+        const double total = del64_sum(m.el + kMaxEl * kElStride, m.nel, C.mass, anc, q, buf);
         if (lane == from) {
           h.x.total = total;
           h.x.pick = -1;
