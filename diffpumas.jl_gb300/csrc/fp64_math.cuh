@@ -12,10 +12,11 @@
 //  - the reciprocal and the reciprocal square root refine the hardware's
 //    approximation by the binomial series of its residual;
 //  - comparisons, minima and uniforms on the bit patterns.
-// All are within 1.5 units in the last place (division: 2) of the exact value
-// on the ranges that the walks use (tested against CUDA's functions); outside
-// them (zeros, negative or subnormal arguments, infinities, NaN) they call
-// CUDA's.
+// Largest errors found against extended precision on the ranges that the walks use,
+// in units of the last place: log 1.8 (below 3/4, where its two parts cancel), exp 1.0,
+// 1/x 0.51, 1/sqrt 1.0, sqrt 1.7, a/b 1.5, 1/(beta gamma) 1.7 (bounds and their reasons:
+// tests/test_gpu_fp64_bounds.py).  Outside (zeros, negative or subnormal arguments,
+// infinities, NaN) log, exp and sqrt call CUDA's; the others are not used there.
 #pragma once
 #include <stdint.h>
 
