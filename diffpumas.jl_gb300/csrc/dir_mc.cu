@@ -358,8 +358,8 @@ struct PathGeo {
     R rho, mx, lE = R(0);  // FP64: the logarithm of the energy serves the whole step
     Loc<R> Li;
     if constexpr (sizeof(R) == 8) {
-      rho = air ? 1.205 * f64::exp((P.B.detector_elevation + s.z) * (-1.0 / 12e3)) : h.rho;
-      lE = f64::log(s.E);
+      rho = air ? 1.205 * f64::exp_fine((P.B.detector_elevation + s.z) * (-1.0 / 12e3)) : h.rho;
+      lE = f64::log_fine(s.E);
       Li = locate_log(m, s.E, lE);
       mx = f64::div(0.01 * at(m, Li, MC_CR), f64::max_pos(rho, air ? 1e-8 : 1e-6));
       if (air) mx = f64::min_pos(mx, f64::div(0.05 * 12e3, f64::max_pos(h.cos_t, 0.05)));

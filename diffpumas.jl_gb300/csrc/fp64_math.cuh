@@ -13,7 +13,8 @@
 //    approximation by the binomial series of its residual;
 //  - comparisons, minima and uniforms on the bit patterns.
 // Largest errors found against extended precision on the ranges that the walks use,
-// in units of the last place: log 1.8 (below 3/4, where its two parts cancel), exp 1.0,
+// in units of the last place: log 1.8 (below 3/4, where its two parts cancel), exp 1.0
+// (their fine forms 1.1 and 0.51),
 // 1/x 0.51, 1/sqrt 1.0, sqrt 1.7, a/b 1.5, 1/(beta gamma) 1.7 (bounds and their reasons:
 // tests/test_gpu_fp64_bounds.py).  Outside (zeros, negative or subnormal arguments,
 // infinities, NaN) log, exp and sqrt call CUDA's; the others are not used there.
@@ -43,29 +44,39 @@ __device__ __forceinline__ double widen(double d) { return d; }
 
 // log x, x normal and positive: 10 FP64 instructions.  x = 2^k m with m / c in
 // [1 - 2^-9, 1 + 2^-9] of the table's c; c = 1 around x = 1, where the result
-// is the polynomial alone.
-__device__ __forceinline__ double log(double x) {
+// is the polynomial alone.  FINE: 11, the sum of the tabulated parts being exact.
+template <bool FINE>
+__device__ __forceinline__ double log_by_table(double x) {
   const int hi = hi32(x);
   if (uint32_t(hi - 0x00100000) >= 0x7fe00000u) return ::log(x);
   const int k = ((hi + 0x00080800) >> 20) - 1023;
-  const double2 t = kLogTab[((hi & 0xfffff) + 0x800) >> 12];
+  const int j = ((hi & 0xfffff) + 0x800) >> 12;
+  const double2 t = FINE ? kLogFine[j] : kLogTab[j];
   const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
   const double r = fma(m, t.x, -1.0);
   const double p = fma(r, fma(r, fma(r, fma(r, -1.0 / 6.0, 0.2), -0.25), 1.0 / 3.0), -0.5);
-  return fma(from_int(k), 0.6931471805599453, t.y) + fma(r * r, p, r);
+  const double kd = from_int(k), q = fma(r * r, p, r);
+  if (FINE) return fma(kd, 0.6931471805598903, t.y) + fma(kd, 5.497923018708371e-14, q);
+  return fma(kd, 0.6931471805599453, t.y) + q;
 }
+__device__ __forceinline__ double log(double x) { return log_by_table<false>(x); }
+__device__ __forceinline__ double log_fine(double x) { return log_by_table<true>(x); }
 
 // exp x: 10 FP64 instructions; x = (128 k + j) log 2 / 128 + r, |r| <= log 2 / 256.
-__device__ __forceinline__ double exp(double x) {
+// FINE: 11, with the table's rounding.
+template <bool FINE>
+__device__ __forceinline__ double exp_by_table(double x) {
   if (uint32_t(hi32(x) & 0x7fffffff) >= 0x40862000u) return ::exp(x);  // |x| >= 708
   const double s = fma(x, 184.6649652337873, 6755399441055744.0);  // 1.5 2^52: nearest integer
   const int n = __double2loint(s);
   const double d = s - 6755399441055744.0;
   const double r = fma(d, -1.2864023111638346e-14, fma(d, -0.005415212348111709, x));
   const double p = fma(r, fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
-  const double t = kExpTab[n & 127], y = fma(t, r * p, t);
+  const double t = kExpTab[n & 127], y = FINE ? t + fma(t, r * p, kExpLow[n & 127]) : fma(t, r * p, t);
   return __hiloint2double(hi32(y) + ((n >> 7) << 20), __double2loint(y));
 }
+__device__ __forceinline__ double exp(double x) { return exp_by_table<false>(x); }
+__device__ __forceinline__ double exp_fine(double x) { return exp_by_table<true>(x); }
 
 // 1 / x for normal x whose reciprocal is normal: 3 FP64 instructions.
 __device__ __forceinline__ double rcp(double x) {
