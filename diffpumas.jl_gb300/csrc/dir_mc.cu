@@ -136,10 +136,13 @@ __device__ __forceinline__ int dir_of(const int64_t* smp, long n_dirs, long i) {
 
 // Grammage of every direction's cells and rock, one warp each: what a history's
 // cost bucket follows.  Longest first, a warp's lanes hold histories of similar
-// length and the short ones fill the end of the launch: mixed, 512 directions of 512
-// samples 26.2 -> 23.5 ms, of 2000 79.6 -> 69.5, 64 of 500 10.1 -> 9.0 ms against index
-// order; FP64, 64 of 6000 108 -> 100 ms, 256 of 512 47.1 -> 41.6, but 64 of 500 (one
-// history for most lanes) 18.3 -> 19.5.
+// length and the short ones fill the end of the launch.  Calls, index order against
+// longest first: under 600 m, 1 MeV to 10^9 GeV, mixed 64 directions of 500 samples 13.1
+// -> 11.1 ms, 256 of 512 19.4 -> 17.3, 64 of 6000 33.7 -> 30.7; FP64 64 of 500 49.3 ->
+// 43.1, 256 of 512 114.7 -> 104.6.  Under 150 m from 1 GeV on the lengths differ less, and
+// it gives or takes a few percent: FP64 16 of 500 11.6 -> 10.6 ms, 64 of 6000 109.4 ->
+// 101.1, but 64 of 500 (one history for most lanes) 18.2 -> 19.2; mixed 64 of 6000 15.3 ->
+// 14.4, but 256 of 512 8.5 -> 8.8.  dp_set_mc_shape has the other order.
 __global__ void __launch_bounds__(256) dir_grammage_kernel(const __grid_constant__ DirParams P) {
   const long d = (blockIdx.x * long(blockDim.x) + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -460,11 +463,9 @@ __global__ void __launch_bounds__(T, 1) dir_kernel(const __grid_constant__ DirPa
   __syncthreads();
   PathGeo<R> geo{P, meds};
   float* coop = reinterpret_cast<float*>(smem + dir_coop_offset<R>(P));
-  transport_histories<R, PHASE>(geo, P.C, P.counter,
-                                               static_cast<DirHandoff<R>*>(P.queue), coop,
-                                               P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
-                                               PHASE == 0 ? P.order0 : P.order1,
-                                               ((P.sync >> PHASE) & 1) != 0);
+  transport_histories<R, PHASE>(geo, P.C, P.counter, static_cast<DirHandoff<R>*>(P.queue), coop,
+                                P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
+                                PHASE == 0 ? P.order0 : P.order1, ((P.sync >> PHASE) & 1) != 0);
 }
 
 // Contribution 2 w_i w flux_gccly(cos zenith, E, q) of every ended history

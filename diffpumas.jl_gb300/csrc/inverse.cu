@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads) cg_apply_kernel(const double* p, con
   block_part(s, sh, part);
 }
 // x += a p, r -= a Ap, z = r iprec with a = r.z / p.Ap, and the block partials of
-// the new r . z (same traversal as above).  Every block sums the 304 partials of
+// the new r . z (pairs of cells, grid stride).  Every block sums the 304 partials of
 // p.Ap for itself, half a microsecond in place of a launch of one block (as the
 // direction does below): ten iterations of 10^6 cells' Gauss-Newton 37.5 -> 36.9 ms.
 __global__ void __launch_bounds__(kThreads) cg_step_dot_kernel(const double* rz, const double* part_pAp,

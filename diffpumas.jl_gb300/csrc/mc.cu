@@ -676,18 +676,14 @@ __global__ void __launch_bounds__(T, 1) mc_kernel(const __grid_constant__ McPara
   if constexpr (POR) {
     const Med<R>& porous = meds[2];
     SlabGeoP<R> geo{P, rock, air, porous};
-    transport_histories<R, PHASE>(geo, P.C, P.counter,
-                                                 static_cast<HandoffP<R>*>(P.queue), coop,
-                                                 P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
-                                                 PHASE == 0 ? P.order0 : P.order1,
-                                                 ((P.sync >> PHASE) & 1) != 0);
+    transport_histories<R, PHASE>(geo, P.C, P.counter, static_cast<HandoffP<R>*>(P.queue), coop,
+                                  P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
+                                  PHASE == 0 ? P.order0 : P.order1, ((P.sync >> PHASE) & 1) != 0);
   } else {
     SlabGeo<R> geo{P, rock, air};
-    transport_histories<R, PHASE>(geo, P.C, P.counter,
-                                                 static_cast<Handoff<R>*>(P.queue), coop,
-                                                 P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
-                                                 PHASE == 0 ? P.order0 : P.order1,
-                                                 ((P.sync >> PHASE) & 1) != 0);
+    transport_histories<R, PHASE>(geo, P.C, P.counter, static_cast<Handoff<R>*>(P.queue), coop,
+                                  P.coop_stride, P.coop_kmax, P.coop_kc, P.coop_nel,
+                                  PHASE == 0 ? P.order0 : P.order1, ((P.sync >> PHASE) & 1) != 0);
   }
 }
 

@@ -131,7 +131,7 @@ __device__ __forceinline__ long next_history(unsigned long long* counter) {
 
 // First hand-out of a launch: the place in the hand-out order of the history that
 // this thread starts with (n or more: none); the counter then deals from
-// deal_first(n) on.  Fewer histories than lanes are spread over all warps of the
+// deal_first() on.  Fewer histories than lanes are spread over all warps of the
 // grid, first one warp of every CTA, then the next, and lanes are filled once every
 // warp has one: a lane alone in its warp costs the FP64 pipe as much as a full warp
 // (64 cycles per instruction, measured) and FP32 little, but a history's divergent

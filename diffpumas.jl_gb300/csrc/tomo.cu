@@ -23,9 +23,9 @@
 //    exponents in FP32; the node flux integral is accumulated in FP64.
 // Adjoint: a reverse sweep over the segment list carries
 // lambda_k = d log(flux)/d E_k; d flux/d rho_k = flux lambda_k dE_k/dY_k L_k.
-// Lanes are reduced per segment by a fixed tree: one Jacobian entry per segment.  J^T r = per-cell sums over the precomputed CSC permutation, each
-// bucket ordered by entry index -- no floating-point atomics, bitwise
-// reproducible.
+// Lanes are reduced per segment by a fixed tree: one Jacobian entry per segment.
+// J^T r = per-cell sums over the precomputed CSC permutation, each bucket ordered by
+// entry index -- no floating-point atomics, bitwise reproducible.
 #include <math_constants.h>
 
 #include <algorithm>
@@ -1625,7 +1625,8 @@ extern "C" int dp_tomo_eval_noalloc_dev(dp_ctx* ctx, const dp_physics* ph, const
   const size_t smem = size_t(2 * kNC32) * P.ld32 * 4 + size_t(kWarps) * P.seg_cap * 3 * 4 +
                       size_t(P.n_nodes) * sizeof(NodeInit);
   if (smem > 220 * 1024)
-    return fail(ctx, DP_ERR_ARG, "energy grid too large, ray too long or too many nodes for the allocation-free form");
+    return fail(ctx, DP_ERR_ARG,
+                "energy grid too large, ray too long or too many nodes for the allocation-free form");
   const long blocks = std::min<long>((pa->n_rays + kWarps - 1) / kWarps, 152L * 16);
   const bool adj = cot != nullptr;
   if (adj) {
