@@ -504,7 +504,7 @@ static int launch(dp_ctx* ctx, CsdaParams& P, const dp_physics* ph32 = nullptr) 
   int per_sm = 0, n_sm = 0;
   // (grids of more than 720 nodes)
   if (ph32 && smem > kSmemDefault)
-    DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(csda32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    DP_CHECK_CUDA(ctx, allow_smem(ctx, csda32_kernel, 64));
   if (ph32)
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, csda32_kernel, threads,
                                                                      smem));

@@ -533,8 +533,7 @@ int dir_device(dp_ctx* ctx, dp_dir_media* M, int precision, dp_dir_media::Dev** 
 template <class R, int PHASE, int T>
 int dir_phase(dp_ctx* ctx, const DirParams& P, size_t smem) {
   const int threads = T;
-  DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(dir_kernel<R, PHASE, T>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  DP_CHECK_CUDA(ctx, allow_smem(ctx, dir_kernel<R, PHASE, T>));
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(dir_kernel<R, PHASE, T>,
                                           cudaFuncAttributePreferredSharedMemoryCarveout,
                                           carveout_percent(ctx->device, smem)));

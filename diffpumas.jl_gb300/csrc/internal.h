@@ -103,6 +103,15 @@ int cuda_fail(dp_ctx* ctx, cudaError_t e, const char* where);
 // temporaries of the MC and plain kernels, 1 Jacobian values of an
 // evaluation, 2 device copies of host inputs, 3 one-shot ray paths.
 void* scratch(dp_ctx* ctx, size_t bytes, int slot = 0);
+// Lets `kernel` ask for all of a block's shared memory less `own` bytes that it declares
+// itself.  Always the same value: the setting is the process's, and one that followed the
+// launch could be lowered by another thread between the two (a failed launch).
+template <class K>
+cudaError_t allow_smem(const dp_ctx* ctx, K* kernel, int own = 0) {
+  int most = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - own);
+}
 // Stochastic run_backward_mc on single-material rock and air media (one line
 // of sight, FP64 or mixed precision per p->precision); fills flux, sigma and
 // the flagged-history count of *res.  Returns DP_ERR_DOMAIN / DP_ERR_STATE

@@ -970,8 +970,7 @@ namespace {
 template <class R, int PHASE, int T, bool POR>
 int launch_phase(dp_ctx* ctx, McParams& P, size_t smem) {
   const int threads = T;
-  DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(mc_kernel<R, PHASE, T, POR>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  DP_CHECK_CUDA(ctx, allow_smem(ctx, mc_kernel<R, PHASE, T, POR>));
   DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(mc_kernel<R, PHASE, T, POR>,
                                           cudaFuncAttributePreferredSharedMemoryCarveout,
                                           carveout_percent(ctx->device, smem)));

@@ -1124,7 +1124,7 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
     while (!fits(T_NCOL) && !fits(T_SEGCOL) && warps > 1) warps /= 2;
     if (smem > most) return fail(ctx, DP_ERR_ARG, "energy grid too large or ray too long for the FP64 kernel");
     auto kernel = adj ? eval64_kernel<true> : eval64_kernel<false>;
-    DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    DP_CHECK_CUDA(ctx, allow_smem(ctx, kernel, 64));
     DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem));
     blocks = std::min<long>((pa->n_rays + warps - 1) / warps, long(std::max(per_sm, 1)) * n_sm);
   }
@@ -1180,7 +1180,7 @@ static int eval_core(dp_ctx* ctx, const dp_physics* ph, const dp_paths* pa, cons
       ++ctx->launches;
       P.node0 = out;
       auto kernel = adj ? eval32_kernel<true, true> : eval32_kernel<false, true>;
-      DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      DP_CHECK_CUDA(ctx, allow_smem(ctx, kernel, 64));
       kernel<<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);
     } else if (adj) {
       eval32_kernel<true><<<int(blocks), kWarps * 32, smem, ctx->stream>>>(P);

@@ -212,8 +212,7 @@ int run(dp_ctx* ctx, const dp_physics* ph, const dp_csda_config* c, const dp_csd
   const size_t smem = mixed ? 16 + size_t(wt::kSlots) * P.col_bytes * 3 / 2 : bytes64(P.staged);
   const int threads = mixed ? wt::kThreads : wt64::kThreads;
   auto kernel = mixed ? wt32::wtomo_kernel : wt64::wtomo_kernel;
-  DP_CHECK_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(smem)));
+  DP_CHECK_CUDA(ctx, allow_smem(ctx, kernel));
   int per_sm = 0, n_sm = 0;
   DP_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   DP_CHECK_CUDA(ctx, cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
