@@ -50,3 +50,27 @@ def test_directions():
         out = run(n)
         for k in ("contrib", "status", "final"):
             np.testing.assert_array_equal(out[k], ref[k][:n])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_few_histories_are_not_ordered(precision):
+    """As many histories as multiprocessors or fewer: the launches of index order."""
+    import dpgpu as dp
+    import torch
+    phys = dp.create_physics(materials=(dp.STANDARD_ROCK, dp.AIR, dp.WATER))
+    cfg, site = dp.MaterialConfig(1, 3, 2, -1, 2650.0, 1000.0, 0.0, 0.0), dp.SiteConfig(963.0, 1200.0)
+    mats, dens = dp.build_cell_properties_for_mc(phys, np.zeros(2, bool), np.array([0.1, 0.3]), cfg)
+    path = dp.DirectionalPath(20.0, 0.0, [dp.CellSegment(1, 1.5), dp.CellSegment(2, 1.0)], 0.0, 0.0, 2.0, 50.0, True)
+    sms, lib, before = torch.cuda.get_device_properties(0).multi_processor_count, dp.load(), dp.get_mc_shape(phys.ctx, "dir", precision)
+    try:
+        for n, more in ((1, False), (sms, False), (sms + 1, True)):
+            batch = dp.DirBatch(phys, cfg, site, [path], mats, dens, None, n_samples=n, energy_min=0.5, energy_max=1e4)
+            launches = []
+            for order in (0, 1):
+                dp.set_mc_shape(phys.ctx, "dir", precision, order=order)
+                k = lib.dp_launch_count(phys.ctx.h)
+                batch.run(5, precision=precision)
+                launches.append(lib.dp_launch_count(phys.ctx.h) - k)
+            assert (launches[0] > launches[1]) == more, (n, launches)
+    finally:
+        dp.set_mc_shape(phys.ctx, "dir", precision, order=before["order"])
